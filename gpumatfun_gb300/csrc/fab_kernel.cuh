@@ -1141,80 +1141,155 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
 // back substitution of a general right-hand side: with the bottom-up Schur
 // complements g_q = (alpha_q - s_q) - beta_{q+1} (beta_{q+1} / g_{q+1}), the
 // solution is y_0 = rhs / g_0 and y_q = -beta_q y_{q-1} / g_q.
-// One thread per system (the recurrence is serial in q; neighbouring lanes
-// take neighbouring contour nodes of the same alpha/beta), complex FP64.
-// Scaling: 1/g is Smith's complex reciprocal (R. L. Smith, "Algorithm 116:
-// Complex division", CACM 5(8), 1962), which never forms |g|^2, and the
-// Schur update multiplies beta by (beta / g) instead of forming beta^2, so
-// entries of T up to ~1e300 and down to ~1e-300 neither overflow nor
-// underflow.  The reciprocals 1/g_q are kept in the tri scratch for the
-// top-down sweep.
+// The recurrence is serial in q; neighbouring lanes take neighbouring contour
+// nodes of the same alpha/beta, complex FP64.
+// Scaling: 1/g is formed from g scaled by the power of two that brings its
+// larger component into [1, 2) (pair_recip), and the Schur update multiplies
+// beta by (beta / g) instead of forming beta^2, so entries of T up to ~1e300
+// and down to ~1e-300 neither overflow nor underflow.
+//
+// What bounds it: FP64 issue.  A warp's FP64 instruction holds its scheduler
+// for 64 cycles on GB300 whatever its active lanes and whether or not it
+// depends on the one before, so the time of a system is its FP64 instruction
+// count per entry.  Hence:
+//   - two lanes per system, one for the real and one for the imaginary part:
+//     one instruction does both parts of every complex operation;
+//   - one cubic Newton reciprocal instead of the two divisions of Smith's
+//     formula on both sides of a branch, and scaling by powers of two on the
+//     integer pipe;
+//   - the top-down sweep multiplies by t_q = beta_q / g_q, which the bottom-up
+//     sweep has formed anyway and keeps in the tri scratch;
+//   - alpha, beta, shifts and t_q are loaded kTriU entries ahead (two: the
+//     engine's kernels have 40 to 64 registers; m = 453 345 us, four 387 us);
+//   - the warps' systems are spread over the blocks, one warp per SM first.
+// Against one thread per system with Smith's reciprocal (phase times):
+// m = 60 120 -> 72 us, m = 453 1010 -> 345 us, 24 problems x 4 right-hand
+// sides of m = 32 419 -> 62 us.
+constexpr int kTriU = 2;
 
-// 1/(a + ib) by Smith's algorithm: the ratio of the smaller to the larger
-// component keeps every intermediate within the range of the inputs.
-__device__ __forceinline__ void smith_recip(double a, double b, double& rr, double& ri) {
-  if (fabs(a) >= fabs(b)) {
-    const double t = b / a;
-    const double inv = 1.0 / (a + b * t);
-    rr = inv;
-    ri = -t * inv;
-  } else {
-    const double t = a / b;
-    const double inv = 1.0 / (a * t + b);
-    rr = t * inv;
-    ri = -inv;
-  }
+// x * 2^(-k) by exponent arithmetic: exact while x and the result are normal
+// numbers, 0 below that (the callers' results stay below the largest number).
+__device__ __forceinline__ double scale_exp2(double x, int k) {
+  const int hi = __double2hiint(x);
+  const int ex = (hi >> 20) & 0x7ff;
+  return ex > max(k, 0) ? __hiloint2double(hi - (k << 20), __double2loint(x)) : 0.0;
+}
+
+// This lane's component of 1/(a + ib), x being this lane's component (even
+// lanes a, odd lanes b).  g is scaled by 2^-e, e the exponent of its larger
+// component, so that |g|^2 lies in [1, 8); its reciprocal takes one cubically
+// convergent Newton step r (1 + h + h^2), h = 1 - d r, from the FP32
+// reciprocal instruction, whose error of about 2^-22 becomes 2^-66 before
+// rounding.
+__device__ __forceinline__ double pair_recip(double x) {
+  const unsigned full = 0xffffffffu;
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
+  const int em = max(ex, __shfl_xor_sync(full, ex, 1));
+  const int k = em - 1023;
+  const double xs = em == 0x7ff ? x : scale_exp2(x, k);   // Inf and NaN pass through as they are
+  const double sq = xs * xs;
+  const double d = sq + __shfl_xor_sync(full, sq, 1);
+  float rf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"((float)d));
+  const double r0 = (double)rf;
+  const double h = fma(-d, r0, 1.0);
+  const double r = fma(r0, fma(h, h, h), r0);
+  const double y = em == 0x7ff ? xs * r : scale_exp2(xs * r, k);
+  return (threadIdx.x & 1) ? -y : y;
 }
 
 template <int R>
 __device__ void phase_trisolve(const KParams& kp, const Ctx& c) {
   const int m = kp.m, C = kp.C;
   const int np = kp.nprob > 0 ? kp.nprob : 1;
-  for (long long sys = c.gt(); sys < (long long)np * R * C; sys += c.tt()) {
+  const long long nsys = (long long)np * R * C;
+  const unsigned full = 0xffffffffu;
+  const bool im = threadIdx.x & 1;
+  // warp w of block b takes systems 16 (w G + b) + lane / 2; lanes past the
+  // last system repeat it without storing, so that every shuffle is full
+  for (long long s0 = 16LL * ((long long)c.warp() * c.G + c.b()); s0 < nsys; s0 += c.tt() / 2) {
+    const long long sl = s0 + (c.lane() >> 1);
+    const bool act = sl < nsys;
+    const long long sys = act ? sl : nsys - 1;
     // sys = (p R + r) C + j for problem p, right-hand side r, node j
     const long long rr = sys / C;
     const int j = (int)(sys % C);
     const long long p = rr / R;
     const int r = (int)(rr % R);
     const int me = kp.meff[rr];
+    int mew = me;   // the warp's largest m_eff: its loops' common length
+    for (int o = 16; o > 0; o >>= 1) mew = max(mew, __shfl_xor_sync(full, mew, o));
     const double* __restrict__ al = kp.aabb + (long long)(m + 1) * (2 * R * p + r);
     const double* __restrict__ be = kp.aabb + (long long)(m + 1) * (2 * R * p + R + r);
-    const double* __restrict__ sh = kp.shifts + 2LL * m * sys;
-    double* __restrict__ ig = kp.tri + 4LL * m * sys;  // 1/g_q (re, im)
-    double* __restrict__ yr = kp.Yr + (long long)m * sys;
-    double* __restrict__ yi = kp.Yi + (long long)m * sys;
-    const double b0 = be[0];
-    const double wr = kp.wts[2LL * C * rr + j], wi = kp.wts[2LL * C * rr + C + j];
-    double igr = 0.0, igi = 0.0;   // 1/g_{q+1}
-#pragma unroll 4
-    for (int q = me - 1; q >= 0; --q) {
-      const double bq = q + 1 < me ? be[q + 1] : 0.0;
-      // beta^2 / g_{q+1} as beta (beta / g_{q+1})
-      const double gr = (al[q] - sh[2 * q]) - bq * (bq * igr);
-      const double gi = -sh[2 * q + 1] - bq * (bq * igi);
-      smith_recip(gr, gi, igr, igi);
-      ig[2 * q] = igr;
-      ig[2 * q + 1] = igi;
+    const double* __restrict__ sh = kp.shifts + 2LL * m * sys + (im ? 1 : 0);
+    double* ts = kp.tri + 4LL * m * sys;   // beta_q / g_q (q >= 1) and 1/g_0, (re, im)
+    double* __restrict__ y = (im ? kp.Yi : kp.Yr) + (long long)m * sys;
+    double t = 0.0, bn = 0.0;   // t_{q+1} and beta_{q+1} of this system
+    double la[kTriU], lb[kTriU], ls[kTriU];
+    auto load = [&](int q0) {
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) {
+        const int q = q0 - u;
+        const bool in = q >= 0 && q < me;
+        la[u] = in && !im ? al[q] : 0.0;
+        lb[u] = in ? be[q] : 0.0;
+        ls[u] = in ? sh[2 * q] : -1.0;
+      }
+    };
+    load(mew - 1);
+    for (int q0 = mew - 1; q0 >= 0; q0 -= kTriU) {
+      double ca[kTriU], cb[kTriU];
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) { ca[u] = la[u] - ls[u]; cb[u] = lb[u]; }
+      load(q0 - kTriU);
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) {
+        const int q = q0 - u;
+        if (q < 0) break;
+        // Schur complement: beta^2 / g_{q+1} as beta (beta / g_{q+1})
+        const double ig = pair_recip(fma(-bn, t, ca[u]));
+        if (q < me) {
+          bn = cb[u];
+          t = q > 0 ? bn * ig : ig;
+          if (act) ts[2 * q + (im ? 1 : 0)] = t;
+        }
+      }
     }
-    // y_0 = rhs * (1/g_0), rhs = -(beta0 w)
-    double y_r = 0.0, y_i = 0.0;
-    if (me > 0) {
-      const double xr = -(b0 * wr), xi = -(b0 * wi);
-      y_r = xr * ig[0] - xi * ig[1];
-      y_i = xr * ig[1] + xi * ig[0];
-      yr[0] = y_r;
-      yi[0] = y_i;
+    // y_0 = rhs / g_0, rhs = -(beta0 w); y_q = -(beta_q / g_q) y_{q-1}
+    double yo = 0.0;
+    {
+      const double b0 = be[0];
+      const double xr = -(b0 * kp.wts[2LL * C * rr + j]), xi = -(b0 * kp.wts[2LL * C * rr + C + j]);
+      const double to = __shfl_xor_sync(full, t, 1);
+      // re: xr tr - xi ti; im: xr ti + xi tr
+      if (me > 0) yo = im ? xr * t + xi * to : xr * t - xi * to;
+      if (act && me > 0) y[0] = yo;
     }
-#pragma unroll 4
-    for (int q = 1; q < me; ++q) {
-      const double tr = -be[q] * y_r, ti = -be[q] * y_i;
-      const double gr = ig[2 * q], gi = ig[2 * q + 1];
-      y_r = tr * gr - ti * gi;
-      y_i = tr * gi + ti * gr;
-      yr[q] = y_r;
-      yi[q] = y_i;
+    __syncwarp();   // ts written by the pair's other lane
+    const double2* tv = reinterpret_cast<const double2*>(ts);
+    double2 lt[kTriU];
+#pragma unroll
+    for (int u = 0; u < kTriU; ++u)
+      if (1 + u < me) lt[u] = tv[1 + u];
+    for (int q0 = 1; q0 < mew; q0 += kTriU) {
+      double2 ct[kTriU];
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) ct[u] = lt[u];
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u)
+        if (q0 + kTriU + u < me) lt[u] = tv[q0 + kTriU + u];
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) {
+        const int q = q0 + u;
+        if (q >= mew) break;
+        // re: ty yi - tx yr; im: -ty yr - tx yi
+        const double other = __shfl_xor_sync(full, yo, 1);
+        yo = fma(im ? -ct[u].y : ct[u].y, other, -(ct[u].x * yo));
+        if (act && q < me) y[q] = yo;
+      }
     }
-    for (int q = me; q < m; ++q) { yr[q] = 0.0; yi[q] = 0.0; }
+    if (act)
+      for (int q = me; q < m; ++q) y[q] = 0.0;
   }
 }
 
@@ -1225,7 +1300,8 @@ __device__ void phase_coef(const KParams& kp, const Ctx& c) {
   const int m = kp.m, C = kp.C, d1 = kp.d + 1;
   const int np = kp.nprob > 0 ? kp.nprob : 1;
   const long long total = (long long)np * R * d1 * m;
-  for (long long t = c.gt(); t < total; t += c.tt()) {
+  // (warps spread over the blocks: FP64 issue is per scheduler)
+  for (long long t = 32LL * ((long long)c.warp() * c.G + c.b()) + c.lane(); t < total; t += c.tt()) {
     // t = (rr d1 + i) m + q with rr = p R + r
     const int q = (int)(t % m);
     const int i = (int)((t / m) % d1);
@@ -1234,6 +1310,7 @@ __device__ void phase_coef(const KParams& kp, const Ctx& c) {
     const double* gr = kp.gs_re + (long long)d1 * C * p;
     const double* gi = kp.gs_im + (long long)d1 * C * p;
     double acc = 0.0;
+#pragma unroll 8
     for (int j = 0; j < C; ++j) {
       const long long col = rr * C + j;
       acc = fma(gr[i + (long long)d1 * j], kp.Yi[col * m + q], acc);
@@ -1415,12 +1492,18 @@ __device__ bool phase_deflate(const KParams& kp, const Ctx& c, int mode) {
     __shared__ double s_z[256];
     const int kr = k * R;
     for (int t0 = 0; t0 < kr; t0 += 256) {
-      for (int t = t0 + c.tid(); t < kr && t < t0 + 256; t += c.nt()) {
-        double acc = 0.0;
+      // one warp per entry, lanes over the blocks' partials (a thread per entry
+      // walked all G of them in series: 256^2 with 10 modes 34.6 us, 1M-row
+      // grids 40 us of a launch)
+      for (int t = t0 + c.warp(); t < kr && t < t0 + 256; t += c.nw()) {
         const double* p = part_z + (long long)t * G;
-        for (int b = 0; b < G; ++b) acc += p[b];
-        s_z[t - t0] = acc;
-        if (c.b() == 0) kp.Z[t] = acc;
+        double acc = 0.0;
+        for (int b = c.lane(); b < G; b += 32) acc += p[b];
+        acc = warp_sum(acc);
+        if (c.lane() == 0) {
+          s_z[t - t0] = acc;
+          if (c.b() == 0) kp.Z[t] = acc;
+        }
       }
       __syncthreads();
       // pass 2 over this chunk of Z entries (rows by thread stride)

@@ -102,9 +102,9 @@ extern "C" int gm_lin_sys_solves_noalloc(int m, int nrhs, int contour_size, cons
   int* meff_slots = reinterpret_cast<int*>(scratch + 4 * kMaxEntries);
   k_fill_meff<<<1, 32, 0, s>>>(meff, meff_slots, nrhs, m);
   kp.meff = meff_slots;
-  // one thread per system, as in the engine's lin_sys_solves phase
+  // two lanes per system, as in the engine's lin_sys_solves phase
   const int threads = 256;
-  const long long systems = (long long)nrhs * contour_size;
+  const long long systems = 2LL * nrhs * contour_size;
   kp.G = (int)((systems + threads - 1) / threads);
   if (nrhs == 1) k_trisolve_noalloc<1><<<kp.G, threads, 0, s>>>(kp);
   if (nrhs == 2) k_trisolve_noalloc<2><<<kp.G, threads, 0, s>>>(kp);
