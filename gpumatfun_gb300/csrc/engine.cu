@@ -48,9 +48,10 @@ struct gm_engine {
   int scale_exp = 0;             // mixed engine: A stored as A * 2^-scale_exp
   unsigned long long epoch = 0;  // launch counter (progress-flag epochs)
   double dep_avg = 0.0;          // mean neighbour-list length per block
-  int Gk[9] = {};                // grid size per phase group (co-residency bound)
-  void* kfn[9] = {};
-  size_t smem[9] = {};           // dynamic shared memory per phase group
+  int Gk[6] = {};                // grid size per phase group (co-residency bound)
+  int Tk[6] = {};                // threads per block per phase group
+  void* kfn[6] = {};
+  size_t smem[6] = {};           // dynamic shared memory per phase group
   std::vector<DevBuf> bufs;
   size_t bytes = 0;
   KParams kp{};
@@ -415,7 +416,7 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
   for (int p = 0; p < np; ++p) pb0[p + 1] = pb0[p] + gp[p];
   const int G = pb0[np];
   e->G = G;
-  for (int g = 0; g < 9; ++g) e->Gk[g] = G;   // every phase group
+  for (int& gk : e->Gk) gk = G;   // every phase group
   e->kp.G = G;
   std::vector<int> bs(G + 1, 0), bprob(G, 0);
   for (int p = 0; p < np; ++p) {
@@ -556,10 +557,9 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
   return GM_OK;
 }
 
-// Phase-group kernels (kern_fp64.cu / kern_mixed.cu): 0 lanczos, 1 solves,
-// 2 apply, 3 deflate/update, 4 fused lanczos + solves + apply.
-enum { KGRP_LANCZOS = 0, KGRP_SOLVE = 1, KGRP_APPLY = 2, KGRP_DEFLATE = 3, KGRP_FUSED = 4,
-       KGRP_LANCZOS_MPK = 5, KGRP_FUSED_MPK = 6, KGRP_LANCZOS_RO = 7, KGRP_FUSED_RO = 8, KGRP_N = 9 };
+// Entry points (kern_*.cu): one phase group each.
+enum { KGRP_LANCZOS = 0, KGRP_SOLVE = 1, KGRP_APPLY = 2, KGRP_DEFLATE = 3, KGRP_LANCZOS_MPK = 4, KGRP_LANCZOS_RO = 5,
+       KGRP_N = 6 };
 
 // The dynamic shared memory limit is an attribute of the kernel function,
 // shared by every handle of the process (per device): only ever raise it, so
@@ -628,12 +628,8 @@ void* pick_kernel(int prec, int R, int group, bool l2) {
 #endif
 
 int group_of(int phases) {
-  const int solve = gm::PH_TRISOLVE | gm::PH_COEF;
-  const int defl = gm::PH_DEFLATE | gm::PH_UPDATE_FKPP | gm::PH_UPDATE_FHN;
-  if ((phases & gm::PH_LANCZOS) && (phases & (solve | gm::PH_APPLY))) return KGRP_FUSED;
   if (phases & gm::PH_LANCZOS) return KGRP_LANCZOS;
-  if ((phases & solve) && (phases & gm::PH_APPLY)) return KGRP_FUSED;
-  if (phases & solve) return KGRP_SOLVE;
+  if (phases & (gm::PH_TRISOLVE | gm::PH_COEF)) return KGRP_SOLVE;
   if (phases & gm::PH_APPLY) return KGRP_APPLY;
   return KGRP_DEFLATE;
 }
@@ -654,8 +650,6 @@ int check_sync(gm_engine* e) {
   return map_status(e, e->h_status[0]);
 }
 
-// Launch the persistent kernel with the given phases; slot selects the event
-// pair used for gm_phase_times.
 // NVTX range per engine phase (build_subspace, lin_sys_solves, apply_V,
 // deflate/update, fused solve), visible to Nsight tools and ncu --nvtx; a
 // no-op without a tool attached.
@@ -670,36 +664,35 @@ struct PhaseRange {
   PhaseRange& operator=(const PhaseRange&) = delete;
 };
 
-int launch(gm_engine* e, int phases, int slot) {
-  PhaseRange nvtx_range(slot);
-  // The barrier counter returns to 0 after every completed barrier; it is
-  // reset explicitly only after an aborted launch (gm_set_U clears errors).
+// One launch of the entry point that runs the given phases.
+int launch_group(gm_engine* e, int phases) {
+  // The barrier counters only grow; they are reset explicitly only after an
+  // aborted launch (gm_set_U clears errors).
   KParams kp = e->kp;
   kp.phases = phases;
   void* args[] = {&kp};
   int grp = group_of(phases);
-  if (e->kp.reorth > 0 && (grp == KGRP_LANCZOS || grp == KGRP_FUSED))
-    grp = grp == KGRP_LANCZOS ? KGRP_LANCZOS_RO : KGRP_FUSED_RO;
-  else if (e->kp.mpk && (grp == KGRP_LANCZOS || grp == KGRP_FUSED))
-    grp = grp == KGRP_LANCZOS ? KGRP_LANCZOS_MPK : KGRP_FUSED_MPK;
+  if (e->kp.reorth > 0 && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_RO;
+  else if (e->kp.mpk && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_MPK;
   kp.G = e->Gk[grp];
   if (e->capturing) {
     // A captured launch replays with the same parameters, so the progress
-    // flags are cleared by a memset node before it and a fixed epoch is used.
-    GM_CUDA(e, cudaMemsetAsync(e->kp.prog, 0, sizeof(unsigned long long) * e->G, e->stream));
+    // flags are cleared by a memset node
+    // before it and a fixed epoch is used.
+    if (grp != KGRP_SOLVE && grp != KGRP_DEFLATE)
+      GM_CUDA(e, cudaMemsetAsync(e->kp.prog, 0, sizeof(unsigned long long) * e->G, e->stream));
     kp.epoch = 1;
   } else {
-    GM_CUDA(e, cudaEventRecord(e->ev[slot][0], e->stream));
     kp.epoch = ++e->epoch;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kp.G);
-  cfg.blockDim = dim3(e->threads);
+  cfg.blockDim = dim3(e->Tk[grp]);
   cfg.dynamicSmemBytes = e->smem[grp];
   cfg.stream = e->stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
+  attr[0].val.cooperative = grp != KGRP_SOLVE;   // the solves have no grid barrier
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (e->l2_window) {
@@ -710,7 +703,25 @@ int launch(gm_engine* e, int phases, int slot) {
   cudaError_t st = cudaLaunchKernelExC(&cfg, e->kfn[grp], args);
   if (st != cudaSuccess) return cuda_fail(e, st, "cooperative launch");
   e->launches++;
-  if (e->capturing) return GM_OK;
+  return GM_OK;
+}
+
+// Runs the given phases; slot selects the event pair of gm_phase_times.  A
+// solve is one launch per phase: compiled into one entry point, the phases
+// share its register budget, and the shifted solves' state spilled in the
+// Lanczos passes' 40 to 64 registers and moved their allocation (117^3 with
+// Gram-Schmidt 21.4 ms in one launch, 17.1 ms apart).
+int launch(gm_engine* e, int phases, int slot) {
+  PhaseRange nvtx_range(slot);
+  if (!e->capturing) GM_CUDA(e, cudaEventRecord(e->ev[slot][0], e->stream));
+  int rc = GM_OK;
+  if (group_of(phases) == KGRP_DEFLATE) {
+    rc = launch_group(e, phases);
+  } else {
+    for (int part : {(int)gm::PH_LANCZOS, (int)gm::PH_TRISOLVE, (int)gm::PH_COEF, gm::PH_APPLY | gm::PH_APPLY_SET})
+      if (rc == GM_OK && (phases & part & ~gm::PH_APPLY_SET)) rc = launch_group(e, phases & part);
+  }
+  if (rc || e->capturing) return rc;
   GM_CUDA(e, cudaEventRecord(e->ev[slot][1], e->stream));
   e->ev_used[slot] = true;
   if (e->sync_mode) return check_sync(e);
@@ -930,19 +941,20 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   long long Gmax = 0;
   for (int g = 0; g < KGRP_N; ++g) {
     e->kfn[g] = pick_kernel(e->prec, e->R, g, l2k);
+    if (g == KGRP_SOLVE) continue;   // sized below
     if (!e->kfn[g]) return fail(e, GM_ERR_UNSUPPORTED, "no kernel for nrhs %d", e->R);
-    e->smem[g] = (g == KGRP_LANCZOS || g == KGRP_APPLY || g == KGRP_FUSED || g == KGRP_LANCZOS_MPK ||
-                  g == KGRP_FUSED_MPK || g == KGRP_LANCZOS_RO || g == KGRP_FUSED_RO) ? stage_smem : 0;
+    e->smem[g] = g == KGRP_DEFLATE ? 0 : stage_smem;
+    e->Tk[g] = e->threads;
     if (e->smem[g] > 48 * 1024)
       GM_CUDA(e, raise_smem_limit(e->dev, e->kfn[g], e->smem[g]));
-    const bool ro_grp = g == KGRP_LANCZOS_RO || g == KGRP_FUSED_RO;
-    const bool mpk_grp = g == KGRP_LANCZOS_MPK || g == KGRP_FUSED_MPK;
+    const bool ro_grp = g == KGRP_LANCZOS_RO;
+    const bool mpk_grp = g == KGRP_LANCZOS_MPK;
     if ((ro_grp && a->reorth == 0) || (mpk_grp && !e->mpk_req)) {
       e->Gk[g] = 0;   // never launched
       continue;
     }
     int nb = 0;
-    GM_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e->kfn[g], e->threads, e->smem[g]));
+    GM_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e->kfn[g], e->Tk[g], e->smem[g]));
     if (nb < 1) return fail(e, GM_ERR_UNSUPPORTED, "kernel group %d cannot be resident with %d threads", g, e->threads);
     const int bps = a->blocks_per_sm > 0 ? std::min(a->blocks_per_sm, nb) : nb;
     long long G = (long long)bps * e->nsm;
@@ -954,6 +966,10 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   e->G = (int)Gmax;
   // blocks per problem and the slice partition (sets e->G to the blocks used)
   if ((rc = build_partition(e, csr, slot_rows, slice_off, pslice0, prow0))) return rc;
+  // The shifted solves and the coefficients take few warps, each bound by FP64
+  // issue: spread over the SMs, without grid barriers.
+  e->Gk[KGRP_SOLVE] = 2 * e->nsm;
+  e->Tk[KGRP_SOLVE] = gm::kSolveThreads;
   e->kp.dep_mode = a->sync_policy == 0 ? 1 : 0;
   if (e->kp.mpk) {
     // the level in between lives in dynamic shared memory after the stages;
@@ -962,19 +978,18 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     const size_t su_bytes = (size_t)e->mpk_nmax * e->R * 8;
     const int need = (e->G + e->nsm - 1) / e->nsm;
     bool fits = true;
-    for (int g : {KGRP_LANCZOS_MPK, KGRP_FUSED_MPK}) {
-      const size_t sm = su_off + su_bytes;
-      if (raise_smem_limit(e->dev, e->kfn[g], sm) != cudaSuccess) {
-        cudaGetLastError();
-        fits = false;
-        break;
-      }
+    const int g = KGRP_LANCZOS_MPK;
+    const size_t sm = su_off + su_bytes;
+    if (raise_smem_limit(e->dev, e->kfn[g], sm) != cudaSuccess) {
+      cudaGetLastError();
+      fits = false;
+    } else {
       int nb = 0;
       GM_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e->kfn[g], e->threads, sm));
-      if (nb < need) { fits = false; break; }
+      fits = nb >= need;
     }
     if (fits) {
-      e->smem[KGRP_LANCZOS_MPK] = e->smem[KGRP_FUSED_MPK] = su_off + su_bytes;
+      e->smem[KGRP_LANCZOS_MPK] = su_off + su_bytes;
       e->kp.su_off = (long long)su_off;
     } else {
       e->kp.mpk = 0;   // the two-hop waits stay: correct, slightly more waiting

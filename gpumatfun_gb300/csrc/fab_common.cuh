@@ -320,8 +320,8 @@ struct GridBar {
           unsigned long long t0 = global_timer_ns();
           unsigned spins = 0;
           while (ld_acquire_u64(c64) < target) {
-            if ((++spins & 31u) == 0u) {
-              if (*(volatile int*)status != 0) { ok = 0; break; }
+            if ((++spins & 3u) == 0u) {
+              if ((spins & 31u) == 0u && *(volatile int*)status != 0) { ok = 0; break; }
               if (global_timer_ns() - t0 > timeout_ns) {
                 atomicCAS(status, 0, (int)ST_TIMEOUT);
                 ok = 0;
@@ -378,8 +378,8 @@ struct DepSync {
         unsigned long long start = 0;
         unsigned spins = 0;
         while (ld_acquire_u64(p) < want) {
-          if ((++spins & 31u) == 0) {
-            if (*(volatile int*)status != 0) { ok = 0; break; }
+          if ((++spins & 3u) == 0) {
+            if ((spins & 31u) == 0 && *(volatile int*)status != 0) { ok = 0; break; }
             const unsigned long long now = global_timer_ns();
             if (start == 0) {
               start = now;
@@ -441,48 +441,62 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Block-sum of N values per thread; thread 0 writes out[j * stride] for j < N.
+// Warp sums of N values per lane (N a power of two up to 32), one of them per
+// lane on return: lane l holds the sum of v[packed_index<N>(l)].  Each stage of
+// the xor tree puts two values' halves side by side, so N values take N - 1 +
+// 5 - log2 N additions instead of 5 N; the sums are bit for bit warp_sum's.
+// A warp's FP64 instruction holds its scheduler for 64 cycles, so with four
+// right-hand sides and 48 warps per SM a block sum was 9 us of issue, now 3.
+template <int N>
+__device__ __forceinline__ int packed_index(int lane) {
+  int r = 0;
+#pragma unroll
+  for (int i = 0; (1 << i) < N; ++i) r |= ((lane >> (4 - i)) & 1) << i;
+  return r;
+}
+template <int N>
+__device__ __forceinline__ double warp_sum_packed(const double (&v)[N]) {
+  static_assert(N <= 32 && (N & (N - 1)) == 0, "power of two");
+  const int lane = threadIdx.x & 31;
+  double w[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) w[j] = v[j];
+  int left = N;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (left > 1) {
+      const bool hi = (lane & o) != 0;
+#pragma unroll
+      for (int j = 0; j < N / 2; ++j) {
+        if (j < left / 2) {
+          const double keep = hi ? w[2 * j + 1] : w[2 * j], give = hi ? w[2 * j] : w[2 * j + 1];
+          w[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      left /= 2;
+    } else {
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+    }
+  }
+  return w[0];
+}
+
+// Block-sum of N values per thread, written to out[j * stride] for j < N.
 // Fixed reduction tree, so the result does not depend on timing.
 template <int N>
 __device__ __forceinline__ void block_sum_store(double (&v)[N], double* out, long long stride) {
-  __shared__ double red[32][N > 0 ? N : 1];
+  __shared__ double red[32][N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int j = 0; j < N; ++j) v[j] = warp_sum(v[j]);
-  if (lane == 0) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) red[warp][j] = v[j];
-  }
+  const double s = warp_sum_packed<N>(v);
+  if ((lane & (32 / N - 1)) == 0) red[warp][packed_index<N>(lane)] = s;
   __syncthreads();
   if (warp == 0) {
+    double t[N];
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double t = lane < nw ? red[lane][j] : 0.0;
-      t = warp_sum(t);
-      if (lane == 0) out[j * stride] = t;
-    }
+    for (int j = 0; j < N; ++j) t[j] = lane < nw ? red[lane][j] : 0.0;
+    const double q = warp_sum_packed<N>(t);
+    if ((lane & (32 / N - 1)) == 0) out[packed_index<N>(lane) * stride] = q;
   }
-  __syncthreads();
-}
-
-// Every block computes the same total of G per-block partials for N
-// quantities (partials laid out [N][G]); deterministic fixed order.
-template <int N>
-__device__ __forceinline__ void grid_total(const double* partials, int G, double (&tot)[N]) {
-  __shared__ double s_tot[N > 0 ? N : 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double t = 0.0;
-      for (int b = lane; b < G; b += 32) t += partials[(long long)j * G + b];
-      t = warp_sum(t);
-      if (lane == 0) s_tot[j] = t;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < N; ++j) tot[j] = s_tot[j];
   __syncthreads();
 }
 

@@ -1,6 +1,6 @@
 // The f(A)b engine's persistent kernel.
 //
-// One cooperative launch runs any contiguous subset of the phases
+// One cooperative launch runs a contiguous subset of the phases
 //   LANCZOS -> TRISOLVE -> COEF -> APPLY -> UPDATE_* -> DEFLATE
 // with bounded grid barriers (GridBar) between passes.  The grid is sized so
 // that every block is co-resident (cudaLaunchCooperativeKernel checks it).
@@ -693,19 +693,18 @@ struct LanczosScalars {
   int all_broken;
 };
 
-// Every block sums the G per-block partials (layout [R][G]) in one fixed
+// Every block sums the G per-block partials (layout [N][G]) in one fixed
 // order into dst (shared memory); deterministic and identical in all blocks.
+// One warp per quantity: a lane's additions are a serial chain of FP64 issue
+// slots, 2.4 us for four right-hand sides in one warp.
 template <int N>
 __device__ __forceinline__ void grid_total_smem(const double* partials, int stride, int count, double* dst) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double t = 0.0;
-      for (int b = lane; b < count; b += 32) t += partials[(long long)j * stride + b];
-      t = warp_sum(t);
-      if (lane == 0) dst[j] = t;
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int j = warp; j < N; j += nw) {
+    double t = 0.0;
+    for (int b = lane; b < count; b += 32) t += partials[(long long)j * stride + b];
+    t = warp_sum(t);
+    if (lane == 0) dst[j] = t;
   }
   __syncthreads();
 }
@@ -1154,17 +1153,21 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
 // count per entry.  Hence:
 //   - two lanes per system, one for the real and one for the imaginary part:
 //     one instruction does both parts of every complex operation;
-//   - one cubic Newton reciprocal instead of the two divisions of Smith's
-//     formula on both sides of a branch, and scaling by powers of two on the
-//     integer pipe;
-//   - the top-down sweep multiplies by t_q = beta_q / g_q, which the bottom-up
-//     sweep has formed anyway and keeps in the tri scratch;
+//   - FP64 engine: one cubic Newton reciprocal and scaling by powers of two on
+//     the integer pipe instead of the two divisions of Smith's formula, and a
+//     top-down sweep that multiplies by t_q = beta_q / g_q, which the bottom-up
+//     sweep has formed anyway;
+//   - mixed engine: Smith's formula (R. L. Smith, "Algorithm 116: Complex
+//     division", CACM 5(8), 1962) on the larger and smaller component instead
+//     of on both sides of a branch, operation for operation what one thread
+//     per system computed.  In a time loop X becomes the next U, and FP32
+//     storage turns a last-bit change of U into changes of 1e-8, so the mixed
+//     engine's results keep their bits;
 //   - alpha, beta, shifts and t_q are loaded kTriU entries ahead (two: the
 //     engine's kernels have 40 to 64 registers; m = 453 345 us, four 387 us);
 //   - the warps' systems are spread over the blocks, one warp per SM first.
-// Against one thread per system with Smith's reciprocal (phase times):
-// m = 60 120 -> 72 us, m = 453 1010 -> 345 us, 24 problems x 4 right-hand
-// sides of m = 32 419 -> 62 us.
+// Against one thread per system with Smith's formula on both sides of a branch
+// (FP64 phase times): m = 60 120 -> 72 us, m = 453 1010 -> 345 us.
 constexpr int kTriU = 2;
 
 // x * 2^(-k) by exponent arithmetic: exact while x and the result are normal
@@ -1198,7 +1201,22 @@ __device__ __forceinline__ double pair_recip(double x) {
   return (threadIdx.x & 1) ? -y : y;
 }
 
-template <int R>
+// The same by Smith's formula, which never forms |g|^2: with x the larger and
+// y the smaller component, t = y / x and v = 1 / (x + y t), 1/g is (v, -t v)
+// for a larger real part and (t v, -v) otherwise.
+__device__ __forceinline__ double pair_recip_smith(double g) {
+  const double o = __shfl_xor_sync(0xffffffffu, g, 1);
+  const bool im = threadIdx.x & 1;
+  const double a = im ? o : g, b = im ? g : o;
+  const bool real_big = (__double_as_longlong(a) & 0x7fffffffffffffffll) >= (__double_as_longlong(b) & 0x7fffffffffffffffll);
+  const double x = real_big ? a : b, y = real_big ? b : a;
+  const double t = y / x;
+  const double v = 1.0 / fma(y, t, x);
+  const double tv = t * v;
+  return im ? (real_big ? -tv : -v) : (real_big ? v : tv);
+}
+
+template <int R, bool kSmith>
 __device__ void phase_trisolve(const KParams& kp, const Ctx& c) {
   const int m = kp.m, C = kp.C;
   const int np = kp.nprob > 0 ? kp.nprob : 1;
@@ -1222,9 +1240,10 @@ __device__ void phase_trisolve(const KParams& kp, const Ctx& c) {
     const double* __restrict__ al = kp.aabb + (long long)(m + 1) * (2 * R * p + r);
     const double* __restrict__ be = kp.aabb + (long long)(m + 1) * (2 * R * p + R + r);
     const double* __restrict__ sh = kp.shifts + 2LL * m * sys + (im ? 1 : 0);
-    double* ts = kp.tri + 4LL * m * sys;   // beta_q / g_q (q >= 1) and 1/g_0, (re, im)
+    // kept per entry, (re, im): 1/g_q, or in the FP64 engine beta_q / g_q for q >= 1
+    double* ts = kp.tri + 4LL * m * sys;
     double* __restrict__ y = (im ? kp.Yi : kp.Yr) + (long long)m * sys;
-    double t = 0.0, bn = 0.0;   // t_{q+1} and beta_{q+1} of this system
+    double t = 0.0, bn = 0.0;   // t_{q+1} = beta_{q+1} / g_{q+1} (Smith: 1/g_{q+1}) and beta_{q+1}
     double la[kTriU], lb[kTriU], ls[kTriU];
     auto load = [&](int q0) {
 #pragma unroll
@@ -1247,10 +1266,11 @@ __device__ void phase_trisolve(const KParams& kp, const Ctx& c) {
         const int q = q0 - u;
         if (q < 0) break;
         // Schur complement: beta^2 / g_{q+1} as beta (beta / g_{q+1})
-        const double ig = pair_recip(fma(-bn, t, ca[u]));
+        const double g = fma(-bn, kSmith ? bn * t : t, ca[u]);
+        const double ig = kSmith ? pair_recip_smith(g) : pair_recip(g);
         if (q < me) {
           bn = cb[u];
-          t = q > 0 ? bn * ig : ig;
+          t = !kSmith && q > 0 ? bn * ig : ig;
           if (act) ts[2 * q + (im ? 1 : 0)] = t;
         }
       }
@@ -1262,29 +1282,42 @@ __device__ void phase_trisolve(const KParams& kp, const Ctx& c) {
       const double xr = -(b0 * kp.wts[2LL * C * rr + j]), xi = -(b0 * kp.wts[2LL * C * rr + C + j]);
       const double to = __shfl_xor_sync(full, t, 1);
       // re: xr tr - xi ti; im: xr ti + xi tr
-      if (me > 0) yo = im ? xr * t + xi * to : xr * t - xi * to;
+      const double q1 = xi * to;
+      if (me > 0) yo = fma(xr, t, im ? q1 : -q1);
       if (act && me > 0) y[0] = yo;
     }
     __syncwarp();   // ts written by the pair's other lane
     const double2* tv = reinterpret_cast<const double2*>(ts);
     double2 lt[kTriU];
-#pragma unroll
-    for (int u = 0; u < kTriU; ++u)
-      if (1 + u < me) lt[u] = tv[1 + u];
-    for (int q0 = 1; q0 < mew; q0 += kTriU) {
-      double2 ct[kTriU];
-#pragma unroll
-      for (int u = 0; u < kTriU; ++u) ct[u] = lt[u];
+    double lq[kTriU];   // Smith: beta_q
+    auto load_t = [&](int q0) {
 #pragma unroll
       for (int u = 0; u < kTriU; ++u)
-        if (q0 + kTriU + u < me) lt[u] = tv[q0 + kTriU + u];
+        if (q0 + u < me) {
+          lt[u] = tv[q0 + u];
+          if (kSmith) lq[u] = be[q0 + u];
+        }
+    };
+    load_t(1);
+    for (int q0 = 1; q0 < mew; q0 += kTriU) {
+      double2 ct[kTriU];
+      double cq[kTriU];
+#pragma unroll
+      for (int u = 0; u < kTriU; ++u) { ct[u] = lt[u]; cq[u] = lq[u]; }
+      load_t(q0 + kTriU);
 #pragma unroll
       for (int u = 0; u < kTriU; ++u) {
         const int q = q0 + u;
         if (q >= mew) break;
-        // re: ty yi - tx yr; im: -ty yr - tx yi
-        const double other = __shfl_xor_sync(full, yo, 1);
-        yo = fma(im ? -ct[u].y : ct[u].y, other, -(ct[u].x * yo));
+        if constexpr (kSmith) {
+          // (tr, ti) = -beta_q y_{q-1}; re: tr gr - ti gi; im: ti gr + tr gi
+          const double po = -cq[u] * yo, q1 = __shfl_xor_sync(full, po, 1) * ct[u].y;
+          yo = fma(po, ct[u].x, im ? q1 : -q1);
+        } else {
+          // re: ty yi - tx yr; im: -ty yr - tx yi
+          const double other = __shfl_xor_sync(full, yo, 1);
+          yo = fma(im ? -ct[u].y : ct[u].y, other, -(ct[u].x * yo));
+        }
         if (act && q < me) y[q] = yo;
       }
     }
@@ -1437,7 +1470,7 @@ __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool 
 // Pass 1 (optional time step, update_U.cu:8-16 / update_U_monodomain.cu:8-22)
 // then Z = Q^T Usol; pass 2: U = Usol - Q Z, update = Q (flam o Z), X = 0
 // (lanczos_impl.cu:84-89, update_U.cu:26-38).
-template <int R>
+template <int R, bool kOrdered>
 __device__ bool phase_deflate(const KParams& kp, const Ctx& c, int mode) {
   const long long n = kp.n;
   const int k = kp.k, G = kp.G;
@@ -1492,17 +1525,37 @@ __device__ bool phase_deflate(const KParams& kp, const Ctx& c, int mode) {
     __shared__ double s_z[256];
     const int kr = k * R;
     for (int t0 = 0; t0 < kr; t0 += 256) {
-      // one warp per entry, lanes over the blocks' partials (a thread per entry
-      // walked all G of them in series: 256^2 with 10 modes 34.6 us, 1M-row
-      // grids 40 us of a launch)
-      for (int t = t0 + c.warp(); t < kr && t < t0 + 256; t += c.nw()) {
-        const double* p = part_z + (long long)t * G;
-        double acc = 0.0;
-        for (int b = c.lane(); b < G; b += 32) acc += p[b];
-        acc = warp_sum(acc);
-        if (c.lane() == 0) {
+      if constexpr (kOrdered) {
+        // the mixed engine's U keeps its bits (see phase_trisolve): one thread
+        // per entry adds the blocks in order, 16 loads ahead of the additions
+        for (int t = t0 + c.tid(); t < kr && t < t0 + 256; t += c.nt()) {
+          double acc = 0.0;
+          const double* p = part_z + (long long)t * G;
+          int b = 0;
+          for (; b + 16 <= G; b += 16) {
+            double v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) v[u] = p[b + u];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) acc += v[u];
+          }
+          for (; b < G; ++b) acc += p[b];
           s_z[t - t0] = acc;
           if (c.b() == 0) kp.Z[t] = acc;
+        }
+      } else {
+        // one warp per entry, lanes over the blocks' partials (one thread per
+        // entry, all G of them in series: 256^2 with 10 modes 35 us a launch,
+        // now 27)
+        for (int t = t0 + c.warp(); t < kr && t < t0 + 256; t += c.nw()) {
+          const double* p = part_z + (long long)t * G;
+          double acc = 0.0;
+          for (int b = c.lane(); b < G; b += 32) acc += p[b];
+          acc = warp_sum(acc);
+          if (c.lane() == 0) {
+            s_z[t - t0] = acc;
+            if (c.b() == 0) kp.Z[t] = acc;
+          }
         }
       }
       __syncthreads();
@@ -1554,6 +1607,16 @@ __device__ bool phase_deflate(const KParams& kp, const Ctx& c, int mode) {
 }
 
 // ------------------------------------------------------------------ kernel
+// Phase groups compiled as separate entry points.
+constexpr int KG_LANCZOS = PH_LANCZOS;
+constexpr int KG_SOLVE = PH_TRISOLVE | PH_COEF;
+constexpr int KG_APPLY = PH_APPLY | PH_APPLY_SET;
+constexpr int KG_DEFLATE = PH_DEFLATE | PH_UPDATE_FKPP | PH_UPDATE_FHN;
+
+// Block size of the shifted solves' entry point: few warps per SM, each with
+// registers for the entries loaded ahead (at 40 they spilled).
+constexpr int kSolveThreads = 128;
+
 // PH is the compile-time set of phases this entry point can run (the runtime
 // mask kp.phases selects among them); specialising on it lets the compiler
 // size registers per phase group.
@@ -1579,7 +1642,7 @@ template <class Pol, int R, int PH>
 #ifndef GM_MINB1L2
 #define GM_MINB1L2 2   // one right-hand side, mixed, matrix held in the L2 window (PolMixedL2)
 #endif
-__global__ void __launch_bounds__(GM_MAXT, (R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
+__global__ void __launch_bounds__(PH == KG_SOLVE ? kSolveThreads : GM_MAXT, (PH == KG_SOLVE ? 3 : R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
                                             : (R == 1 ? ((PH & (PH_MPK | PH_REORTH)) ? GM_MINB1X
                                                                                      : (Pol::kL2 ? GM_MINB1L2 : GM_MINB1))
                                                       : GM_MINB))) fab_kernel(KParams kp) {
@@ -1601,7 +1664,7 @@ __global__ void __launch_bounds__(GM_MAXT, (R >= 4 ? ((Pol::kMixed && !(PH & (PH
   }
   if ((PH & PH_TRISOLVE) && (ph & PH_TRISOLVE)) {
     if (!sep()) return;
-    phase_trisolve<R>(kp, c);
+    phase_trisolve<R, Pol::kMixed>(kp, c);
   }
   if ((PH & PH_COEF) && (ph & PH_COEF)) {
     if (!sep()) return;
@@ -1615,15 +1678,9 @@ __global__ void __launch_bounds__(GM_MAXT, (R >= 4 ? ((Pol::kMixed && !(PH & (PH
     const int upd_mode = (ph & PH_UPDATE_FKPP) ? 1 : ((ph & PH_UPDATE_FHN) ? 2 : 0);
     if ((ph & PH_DEFLATE) || upd_mode) {
       if (!sep()) return;
-      if (!phase_deflate<R>(kp, c, upd_mode)) return;
+      if (!phase_deflate<R, Pol::kMixed>(kp, c, upd_mode)) return;
     }
   }
 }
-
-// Phase groups compiled as separate entry points.
-constexpr int KG_LANCZOS = PH_LANCZOS;
-constexpr int KG_SOLVE = PH_TRISOLVE | PH_COEF;
-constexpr int KG_APPLY = PH_APPLY | PH_APPLY_SET;
-constexpr int KG_DEFLATE = PH_DEFLATE | PH_UPDATE_FKPP | PH_UPDATE_FHN;
 
 }  // namespace gm

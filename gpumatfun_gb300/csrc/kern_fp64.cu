@@ -9,11 +9,8 @@ static void* group_ptr(int group) {
     case 1: return (void*)fab_kernel<Pol, R, KG_SOLVE>;
     case 2: return (void*)fab_kernel<Pol, R, KG_APPLY>;
     case 3: return (void*)fab_kernel<Pol, R, KG_DEFLATE>;
-    case 4: return (void*)fab_kernel<Pol, R, KG_LANCZOS | KG_SOLVE | KG_APPLY>;
-    case 5: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_MPK>;
-    case 6: return (void*)fab_kernel<Pol, R, KG_LANCZOS | KG_SOLVE | KG_APPLY | PH_MPK>;
-    case 7: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_REORTH>;
-    case 8: return (void*)fab_kernel<Pol, R, KG_LANCZOS | KG_SOLVE | KG_APPLY | PH_REORTH>;
+    case 4: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_MPK>;
+    case 5: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_REORTH>;
   }
   return nullptr;
 }

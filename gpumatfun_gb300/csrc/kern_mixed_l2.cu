@@ -10,7 +10,6 @@ void* kernel_mixed_l2(int group) {
   switch (group) {
     case 0: return (void*)fab_kernel<PolMixedL2, 1, KG_LANCZOS>;
     case 2: return (void*)fab_kernel<PolMixedL2, 1, KG_APPLY>;
-    case 4: return (void*)fab_kernel<PolMixedL2, 1, KG_LANCZOS | KG_SOLVE | KG_APPLY>;
   }
   return nullptr;
 }

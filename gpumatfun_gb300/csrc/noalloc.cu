@@ -60,7 +60,7 @@ __global__ void k_fill_meff(const int* meff, int* slots, int R, int m) {
 template <int R>
 __global__ void k_trisolve_noalloc(gm::KParams kp) {
   const gm::Ctx c(kp.G);
-  gm::phase_trisolve<R>(kp, c);
+  gm::phase_trisolve<R, false>(kp, c);
 }
 
 }  // namespace
