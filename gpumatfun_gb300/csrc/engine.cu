@@ -25,6 +25,7 @@ namespace gm {
 void* kernel_fp64(int R, int group);
 void* kernel_mixed(int R, int group);
 void* kernel_mixed_l2(int group);
+void* kernel_resident(bool fp64, int R, bool fused);
 }  // namespace gm
 
 namespace {
@@ -48,10 +49,10 @@ struct gm_engine {
   int scale_exp = 0;             // mixed engine: A stored as A * 2^-scale_exp
   unsigned long long epoch = 0;  // launch counter (progress-flag epochs)
   double dep_avg = 0.0;          // mean neighbour-list length per block
-  int Gk[6] = {};                // grid size per phase group (co-residency bound)
-  int Tk[6] = {};                // threads per block per phase group
-  void* kfn[6] = {};
-  size_t smem[6] = {};           // dynamic shared memory per phase group
+  int Gk[8] = {};                // grid size per phase group (co-residency bound)
+  int Tk[8] = {};                // threads per block per phase group
+  void* kfn[8] = {};
+  size_t smem[8] = {};           // dynamic shared memory per phase group
   std::vector<DevBuf> bufs;
   size_t bytes = 0;
   KParams kp{};
@@ -71,6 +72,8 @@ struct gm_engine {
   bool mpk_req = false;          // matrix-powers passes requested
   long long mpk_nmax = 0;        // largest own + halo rows of a block
   std::vector<int> sell_col_host;  // SELL column indices kept for the halo build
+  bool res = false;              // the Lanczos phase keeps the problem on chip (fab_resident.cuh)
+  size_t res_word_bytes = 0;     // its tagged words (one allocation)
   std::vector<double> roww;      // mixed engine: weights of the diagonal compensation (empty = ones)
   bool comp = false;             // mixed engine: diagonal compensation on
   int* row2slot = nullptr;       // device, kept with the entry map: row -> 32 * slice + lane
@@ -320,7 +323,7 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   long long* d_off;
   int rc;
   if ((rc = dupload(e, &d_off, off.data(), off.size()))) return rc;
-  if (e->mpk_req && np == 1 && !(sorted || np > 1)) e->sell_col_host = col;
+  if (np == 1 && !sorted) e->sell_col_host = col;
   // Diagonal compensation of the FP32-stored matrix: row r gets the extra
   // diagonal term c_r = sum_t (a_t 2^-e - fl32(a_t 2^-e)) w_col(t) / w_r, so
   // that the stored operator maps w exactly as A does.  The small eigenvalues
@@ -389,20 +392,142 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   return GM_OK;
 }
 
+// Cost of a slice in the partition: its padded entries plus a per-row cost.
+double slice_cost(const std::vector<long long>& off, long long s) {
+  return (double)(off[s + 1] - off[s]) + 32.0 * 4.0;
+}
+
+// Bounds of G contiguous ranges of slices s0..s1 of about equal cost.
+void balanced_bounds(const std::vector<long long>& off, long long s0, long long s1, int G, int* bs) {
+  double total = 0.0;
+  for (long long s = s0; s < s1; ++s) total += slice_cost(off, s);
+  double acc = 0.0;
+  int b = 0;
+  bs[0] = (int)s0;
+  for (long long s = s0; s < s1; ++s) {
+    const double w = slice_cost(off, s);
+    while (b < G - 1 && acc + 0.5 * w > total * (b + 1) / G) bs[++b] = (int)s;
+    acc += w;
+  }
+  while (b < G - 1) bs[++b] = (int)s1;
+  bs[G] = (int)s1;
+}
+
+// The resident Lanczos phase's partition (fab_resident.cuh): G blocks of nw
+// warps, at most one slice per warp, and per block its halo rows and the
+// columns in block-local numbering.
+struct ResidentPlan {
+  int nw = 0, G = 0;
+  std::vector<int> bs;                  // [G + 1] first slice of each block
+  std::vector<long long> hptr;          // [G + 1]
+  std::vector<int> hrows;
+  std::vector<unsigned short> col;      // per SELL slot entry
+  std::vector<unsigned char> exported;  // per slot: another block references the row
+  int ent = 0, vec = 0;                 // capacities: entries, vector elements per right-hand side
+  size_t bytes = 0;                     // shared memory of the state
+};
+
+// False when the problem has more than 16 slices per SM or a block's local
+// numbering does not fit 16 bits.
+// FP64: equal counts of slices, as few per SM as the SMs allow (FP64 issue
+// bounds the rows of a pass) but at least kResMinSlices: below that a block
+// only adds to every reduction (64 x 64: 5.4 us per step with four slices, 5.6
+// with two, 5.8 with eight, before the integer sums).
+// Mixed: the general path's blocks of 16 warps, for the same sums (a balanced
+// range can hold a slice or two more; up to four are taken).
+constexpr int kResMinSlices = 4;
+bool plan_resident(const gm_engine* e, const Csr& A, const std::vector<long long>& off, ResidentPlan& pl) {
+  const long long nsl = (long long)off.size() - 1;
+  if (nsl < 1 || nsl > 16LL * e->nsm || e->sell_col_host.empty()) return false;
+  const bool mixed = e->prec != GM_FP64;
+  if (mixed) {
+    pl.G = (int)((nsl + 15) / 16);
+  } else {
+    const long long nw = std::max<long long>(kResMinSlices, (nsl + e->nsm - 1) / e->nsm);
+    pl.G = (int)((nsl + nw - 1) / nw);
+  }
+  const int G = pl.G;
+  pl.bs.resize(G + 1);
+  if (mixed) {
+    balanced_bounds(off, 0, nsl, G, pl.bs.data());
+  } else {
+    for (int q = 0; q <= G; ++q) pl.bs[q] = (int)(nsl * q / G);
+  }
+  for (int q = 0; q < G; ++q) {
+    if (pl.bs[q + 1] <= pl.bs[q]) return false;
+    pl.nw = std::max(pl.nw, pl.bs[q + 1] - pl.bs[q]);
+  }
+  if (pl.nw * 32 > gm::kResThreads) return false;
+  const int own_cap = pl.nw * 32;
+  std::vector<int> owner(nsl);
+  for (int q = 0; q < G; ++q)
+    for (int s = pl.bs[q]; s < pl.bs[q + 1]; ++s) owner[s] = q;
+  pl.col.resize(e->sell_col_host.size());
+  pl.exported.assign(nsl * 32, 0);
+  std::vector<unsigned char> reads((size_t)G * G, 0);
+  std::vector<std::vector<int>> halos(G);
+  std::vector<int> seen(e->n, -1);              // last block that met the row in its halo
+  std::vector<unsigned short> local(e->n, 0);   // and its local index there
+  const int* sc = e->sell_col_host.data();
+  for (int q = 0; q < G; ++q) {
+    const int r0 = 32 * pl.bs[q], r1 = (int)std::min<long long>(32LL * pl.bs[q + 1], e->n);
+    std::vector<int>& halo = halos[q];
+    for (long long t = A.ptr[r0]; t < A.ptr[r1]; ++t) {
+      const int c = A.col[t];
+      if ((c < r0 || c >= r1) && seen[c] != q) {
+        seen[c] = q;
+        halo.push_back(c);
+      }
+    }
+    if (own_cap + halo.size() > 60000) return false;
+    std::sort(halo.begin(), halo.end());
+    for (size_t i = 0; i < halo.size(); ++i) {
+      local[halo[i]] = (unsigned short)(own_cap + i);
+      reads[(size_t)q * G + owner[halo[i] / 32]] = 1;
+    }
+    for (int s = pl.bs[q]; s < pl.bs[q + 1]; ++s)
+      for (long long t = off[s]; t < off[s + 1]; t += 32)
+        for (int l = 0; l < 32; ++l) {
+          // padding rows: themselves (slot = row without a permutation)
+          const int c = 32 * s + l < e->n ? sc[t + l] : 32 * s + l;
+          pl.col[t + l] = 32 * s + l >= e->n || (c >= r0 && c < r1) ? (unsigned short)(c - r0) : local[c];
+        }
+    pl.ent = std::max(pl.ent, (int)std::min<long long>(off[pl.bs[q + 1]] - off[pl.bs[q]], 1 << 20));
+  }
+  // a block that is read by another without reading it gets a row of it to
+  // wait for
+  for (int q = 0; q < G; ++q)
+    for (int o = 0; o < G; ++o)
+      if (reads[(size_t)o * G + q] && !reads[(size_t)q * G + o]) halos[q].push_back(32 * pl.bs[o]);
+  pl.hptr.assign(G + 1, 0);
+  for (int q = 0; q < G; ++q) {
+    for (int r : halos[q]) pl.exported[r] = 1;
+    pl.hrows.insert(pl.hrows.end(), halos[q].begin(), halos[q].end());
+    pl.hptr[q + 1] = (long long)pl.hrows.size();
+    pl.vec = std::max(pl.vec, own_cap + (int)halos[q].size());
+  }
+  pl.ent = (pl.ent + 63) & ~63;
+  pl.vec = (pl.vec + 3) & ~3;
+  const size_t vbytes = mixed ? 4 : 8;
+  pl.bytes = (size_t)pl.ent * (vbytes + 2) + (size_t)2 * pl.vec * e->R * 8 + (size_t)32 * e->R * 8 +
+             (mixed ? (size_t)128 * e->R * 12 : 0);
+  return true;
+}
+
 // Static partition of the SELL slices over the G blocks (contiguous ranges
 // balanced by padded entries plus a per-row cost) and, per block, the sorted
 // list of other blocks owning a row that one of its rows references, closed
 // under symmetry (see DepSync in fab_common.cuh).
 int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& rows,
                     const std::vector<long long>& off, const std::vector<long long>& pslice0,
-                    const std::vector<long long>& prow0) {
+                    const std::vector<long long>& prow0, const ResidentPlan& plan) {
   const int np = (int)pslice0.size() - 1;
   // blocks per problem in proportion to its work, at least one, at most one
   // per slice; e->G becomes the total
   std::vector<double> work(np, 0.0);
   std::vector<int> gp(np, 1);
   for (int p = 0; p < np; ++p)
-    for (long long s = pslice0[p]; s < pslice0[p + 1]; ++s) work[p] += (double)(off[s + 1] - off[s]) + 32.0 * 4.0;
+    for (long long s = pslice0[p]; s < pslice0[p + 1]; ++s) work[p] += slice_cost(off, s);
   if (e->G < np) return fail(e, GM_ERR_UNSUPPORTED, "%d problems need at least as many resident blocks (have %d)", np, e->G);
   for (int extra = e->G - np; extra > 0; --extra) {
     int best = -1;
@@ -420,21 +545,10 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
   e->kp.G = G;
   std::vector<int> bs(G + 1, 0), bprob(G, 0);
   for (int p = 0; p < np; ++p) {
-    double total = 0.0;
-    for (long long s = pslice0[p]; s < pslice0[p + 1]; ++s) total += (double)(off[s + 1] - off[s]) + 32.0 * 4.0;
-    double acc = 0.0;
-    int b = 0;
-    const int Gp = gp[p];
-    bs[pb0[p]] = (int)pslice0[p];
-    for (long long s = pslice0[p]; s < pslice0[p + 1]; ++s) {
-      const double w = (double)(off[s + 1] - off[s]) + 32.0 * 4.0;
-      while (b < Gp - 1 && acc + 0.5 * w > total * (b + 1) / Gp) bs[pb0[p] + (++b)] = (int)s;
-      acc += w;
-    }
-    while (b < Gp - 1) bs[pb0[p] + (++b)] = (int)pslice0[p + 1];
-    bs[pb0[p + 1]] = (int)pslice0[p + 1];
+    balanced_bounds(off, pslice0[p], pslice0[p + 1], gp[p], bs.data() + pb0[p]);
     for (int q = pb0[p]; q < pb0[p + 1]; ++q) bprob[q] = p;
   }
+  if (e->res) bs = plan.bs;   // at most one slice per warp
   std::vector<int> owner(e->n, 0);
   for (int q = 0; q < G; ++q)
     for (long long s = bs[q]; s < bs[q + 1]; ++s)
@@ -458,7 +572,7 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
       }
   // Matrix-powers passes: per block the halo rows (referenced by its rows,
   // owned elsewhere), local column indices, and waits over two hops.
-  const bool mpk = e->mpk_req && !e->sell_col_host.empty();
+  const bool mpk = e->mpk_req && !e->res && !e->sell_col_host.empty();
   std::vector<long long> hptr;
   std::vector<int> hrows, lcol;
   if (mpk) {
@@ -554,21 +668,54 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
     e->kp.lcol = d_lcol;
     e->kp.mpk = 1;   // confirmed (or withdrawn) once the shared memory is sized
   }
+  if (e->res) {
+    // one allocation: words (partials at a 128-byte line per block, slice
+    // sums, exchanged rows), then the plan's lists
+    const size_t nr = 2 * (size_t)G * gm::kRedStride;
+    const size_t nss = e->prec == GM_FP64 ? 0 : (size_t)e->nslices * gm::kRedStride;
+    const size_t nw = 2 * (size_t)e->n * e->R;
+    e->res_word_bytes = (nr + nss + nw) * sizeof(ulonglong2);
+    const size_t bp = plan.hptr.size() * sizeof(long long), bh = plan.hrows.size() * sizeof(int),
+                 bc = plan.col.size() * sizeof(unsigned short), bx = plan.exported.size();
+    std::vector<unsigned char> blob(bp + bh + bc + bx);
+    std::memcpy(blob.data(), plan.hptr.data(), bp);
+    if (bh) std::memcpy(blob.data() + bp, plan.hrows.data(), bh);
+    if (bc) std::memcpy(blob.data() + bp + bh, plan.col.data(), bc);
+    std::memcpy(blob.data() + bp + bh + bc, plan.exported.data(), bx);
+    unsigned char* d;
+    if ((rc = dalloc(e, &d, e->res_word_bytes + blob.size()))) return rc;
+    GM_CUDA(e, cudaMemset(d, 0, e->res_word_bytes));   // tag 0 belongs to no launch
+    GM_CUDA(e, cudaMemcpy(d + e->res_word_bytes, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    e->kp.res_red = reinterpret_cast<ulonglong2*>(d);
+    e->kp.res_slice = e->kp.res_red + nr;
+    e->kp.res_words = e->kp.res_slice + nss;
+    d += e->res_word_bytes;
+    e->kp.halo_ptr = reinterpret_cast<const long long*>(d);
+    e->kp.halo_rows = reinterpret_cast<const int*>(d + bp);
+    e->kp.res_col = reinterpret_cast<const unsigned short*>(d + bp + bh);
+    e->kp.res_exp = d + bp + bh + bc;
+    e->kp.res_ent = plan.ent;
+    e->kp.res_vec = plan.vec;
+  }
   return GM_OK;
 }
 
-// Entry points (kern_*.cu): one phase group each.
+// Entry points (kern_*.cu): one phase group each; the resident Lanczos phase
+// also with the rest of a solve.
 enum { KGRP_LANCZOS = 0, KGRP_SOLVE = 1, KGRP_APPLY = 2, KGRP_DEFLATE = 3, KGRP_LANCZOS_MPK = 4, KGRP_LANCZOS_RO = 5,
-       KGRP_N = 6 };
+       KGRP_LANCZOS_RES = 6, KGRP_FUSED_RES = 7, KGRP_N = 8 };
 
 // The dynamic shared memory limit is an attribute of the kernel function,
 // shared by every handle of the process (per device): only ever raise it, so
 // that a handle created later with less shared memory cannot lower the limit
 // under an earlier one.
+// (48 KB are allowed without it, the kernel's static shared memory included,
+// which stays below 16 KB.)
+constexpr size_t kSmemDefault = 32 * 1024;
 cudaError_t raise_smem_limit(int dev, void* kfn, size_t bytes) {
   static std::mutex mu;
   static std::map<std::pair<int, void*>, size_t> set;
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes <= kSmemDefault) return cudaSuccess;
   std::lock_guard<std::mutex> lock(mu);
   size_t& cur = set[{dev, kfn}];
   if (bytes <= cur) return cudaSuccess;
@@ -614,6 +761,7 @@ void window_release(int dev) {
 // right-hand side then runs the SpMV groups compiled for two resident blocks
 // per SM (gm::PolMixedL2, no register spills).
 void* pick_kernel(int prec, int R, int group, bool l2) {
+  if (group >= KGRP_LANCZOS_RES) return gm::kernel_resident(prec == GM_FP64, R, group == KGRP_FUSED_RES);
   if (l2 && R == 1 && prec != GM_FP64) {
     void* k = gm::kernel_mixed_l2(group);
     if (k) return k;
@@ -672,15 +820,19 @@ int launch_group(gm_engine* e, int phases) {
   kp.phases = phases;
   void* args[] = {&kp};
   int grp = group_of(phases);
-  if (e->kp.reorth > 0 && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_RO;
+  if (e->res && (phases & gm::PH_LANCZOS))
+    grp = (phases & gm::PH_APPLY) ? KGRP_FUSED_RES : KGRP_LANCZOS_RES;
+  else if (e->kp.reorth > 0 && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_RO;
   else if (e->kp.mpk && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_MPK;
   kp.G = e->Gk[grp];
   if (e->capturing) {
     // A captured launch replays with the same parameters, so the progress
-    // flags are cleared by a memset node
+    // flags (and the resident phase's words) are cleared by a memset node
     // before it and a fixed epoch is used.
     if (grp != KGRP_SOLVE && grp != KGRP_DEFLATE)
       GM_CUDA(e, cudaMemsetAsync(e->kp.prog, 0, sizeof(unsigned long long) * e->G, e->stream));
+    if (e->res && (phases & gm::PH_LANCZOS))
+      GM_CUDA(e, cudaMemsetAsync(e->kp.res_red, 0, e->res_word_bytes, e->stream));
     kp.epoch = 1;
   } else {
     kp.epoch = ++e->epoch;
@@ -710,12 +862,13 @@ int launch_group(gm_engine* e, int phases) {
 // solve is one launch per phase: compiled into one entry point, the phases
 // share its register budget, and the shifted solves' state spilled in the
 // Lanczos passes' 40 to 64 registers and moved their allocation (117^3 with
-// Gram-Schmidt 21.4 ms in one launch, 17.1 ms apart).
+// Gram-Schmidt 21.4 ms in one launch, 17.1 ms apart).  The resident
+// entry points run one block per SM with registers for all of them.
 int launch(gm_engine* e, int phases, int slot) {
   PhaseRange nvtx_range(slot);
   if (!e->capturing) GM_CUDA(e, cudaEventRecord(e->ev[slot][0], e->stream));
   int rc = GM_OK;
-  if (group_of(phases) == KGRP_DEFLATE) {
+  if ((e->res && (phases & gm::PH_LANCZOS)) || group_of(phases) == KGRP_DEFLATE) {
     rc = launch_group(e, phases);
   } else {
     for (int part : {(int)gm::PH_LANCZOS, (int)gm::PH_TRISOLVE, (int)gm::PH_COEF, gm::PH_APPLY | gm::PH_APPLY_SET})
@@ -922,8 +1075,37 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   const bool stage_l2 = e->prec == GM_FP64 && !e->mpk_req;
   const bool staging = a->col_staging == 2 ||
                        (a->col_staging == 0 && (!use_window || a->val_prefetch == 1 || stage_l2));
+  // Resident Lanczos phase: one block per SM with at most one slice per warp,
+  // the problem on chip between passes.  It is the engine's own choice of a
+  // launch shape: taken only where every launch-shape option is at its
+  // default, for a single unsorted problem without reorthogonalisation that
+  // fits (plan_resident, and shared memory below).  It replaces matrix-powers
+  // passes too, whose point is to halve the passes' waits.  Per Lanczos step,
+  // general path against this one: FP64 64 x 64 12.6 -> 5.0 us, 256 x 256
+  // 13.6 -> 8.6, 128 x 128 with two right-hand sides 18.9 -> 7.1, a 20k-node
+  // disk with two and degree 8 72 -> 22; mixed 256 x 256 with two 19.4 -> 11.9.
+  // Past 16 slices per SM a warp would hold several rows per lane, and the
+  // general path's passes are long enough to hide most of its round trips.
+  ResidentPlan plan;
+  e->res = np == 1 && a->sell_sigma <= 1 && a->reorth == 0 && a->threads_per_block == 0 && a->blocks_per_sm == 0 &&
+           a->max_blocks == 0 && a->sync_policy == 0 && a->col_staging == 0 && a->val_prefetch == 0 &&
+           a->l2_window == 0 && plan_resident(e, csr, slice_off, plan);
   const int stage_cap = staging ? (int)std::min<long long>(max_len, 24) : 0;
-  const size_t stage_smem = stage_cap > 0 ? (size_t)16 * (e->threads / 32) + (size_t)2 * (e->threads / 32) * stage_cap * 128 : 0;
+  auto stage_bytes = [&](int threads) {
+    return stage_cap > 0 ? (size_t)16 * (threads / 32) + (size_t)2 * (threads / 32) * stage_cap * 128 : (size_t)0;
+  };
+  if (e->res) {
+    int optin = 0;
+    GM_CUDA(e, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->dev));
+    // (the kernels' static shared memory stays below 16 KB)
+    if (stage_bytes(plan.nw * 32) + plan.bytes + 16 * 1024 > (size_t)optin) e->res = false;
+  }
+  // The FP64 engine's other groups take the resident block shape too; the
+  // mixed engine's keep the general path's 512 threads and with them the
+  // order of the deflation sums.
+  const int res_threads = e->res ? plan.nw * 32 : e->threads;
+  if (e->res && e->prec == GM_FP64) e->threads = res_threads;
+  const size_t stage_smem = stage_bytes(e->threads);
   e->kp.stage_cap = stage_cap;
   e->kp.pf_vals = 0;
   if (stage_cap > 0 && a->val_prefetch != 2) {
@@ -943,29 +1125,35 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     e->kfn[g] = pick_kernel(e->prec, e->R, g, l2k);
     if (g == KGRP_SOLVE) continue;   // sized below
     if (!e->kfn[g]) return fail(e, GM_ERR_UNSUPPORTED, "no kernel for nrhs %d", e->R);
+    const bool res_grp = g == KGRP_LANCZOS_RES || g == KGRP_FUSED_RES;
     e->smem[g] = g == KGRP_DEFLATE ? 0 : stage_smem;
-    e->Tk[g] = e->threads;
-    if (e->smem[g] > 48 * 1024)
+    e->Tk[g] = res_grp ? res_threads : e->threads;
+    if (res_grp && e->res) {
+      e->kp.res_off = (int)((stage_bytes(res_threads) + 127) & ~(size_t)127);
+      e->smem[g] = e->kp.res_off + plan.bytes;
+    }
+    if (e->smem[g] > kSmemDefault)
       GM_CUDA(e, raise_smem_limit(e->dev, e->kfn[g], e->smem[g]));
     const bool ro_grp = g == KGRP_LANCZOS_RO;
     const bool mpk_grp = g == KGRP_LANCZOS_MPK;
-    if ((ro_grp && a->reorth == 0) || (mpk_grp && !e->mpk_req)) {
+    if ((ro_grp && a->reorth == 0) || (mpk_grp && !e->mpk_req) || (res_grp && !e->res)) {
       e->Gk[g] = 0;   // never launched
       continue;
     }
     int nb = 0;
     GM_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e->kfn[g], e->Tk[g], e->smem[g]));
-    if (nb < 1) return fail(e, GM_ERR_UNSUPPORTED, "kernel group %d cannot be resident with %d threads", g, e->threads);
+    if (nb < 1) return fail(e, GM_ERR_UNSUPPORTED, "kernel group %d cannot be resident with %d threads", g, e->Tk[g]);
     const int bps = a->blocks_per_sm > 0 ? std::min(a->blocks_per_sm, nb) : nb;
     long long G = (long long)bps * e->nsm;
     if (a->blocks_per_sm <= 0) G = std::min(G, want);
     if (a->max_blocks > 0) G = std::min<long long>(G, std::max<long long>(np, a->max_blocks));
+    if (e->res) G = plan.G;   // at most one block per SM
     e->Gk[g] = (int)std::max<long long>(1, G);
     Gmax = Gmax == 0 ? e->Gk[g] : std::min(Gmax, (long long)e->Gk[g]);
   }
   e->G = (int)Gmax;
   // blocks per problem and the slice partition (sets e->G to the blocks used)
-  if ((rc = build_partition(e, csr, slot_rows, slice_off, pslice0, prow0))) return rc;
+  if ((rc = build_partition(e, csr, slot_rows, slice_off, pslice0, prow0, plan))) return rc;
   // The shifted solves and the coefficients take few warps, each bound by FP64
   // issue: spread over the SMs, without grid barriers.
   e->Gk[KGRP_SOLVE] = 2 * e->nsm;
@@ -1768,7 +1956,7 @@ int gm_phase_times(gm_handle h, float* ms) {
 int gm_info(gm_handle h, int64_t* info) {
   if (!h || !info) return GM_ERR_ARG;
   info[0] = h->n; info[1] = h->R; info[2] = h->m; info[3] = h->d; info[4] = h->C; info[5] = h->k;
-  info[6] = h->prec; info[7] = h->G; info[8] = h->threads; info[9] = h->padded;
+  info[6] = h->prec; info[7] = h->G; info[8] = h->Tk[h->res ? KGRP_FUSED_RES : KGRP_LANCZOS]; info[9] = h->padded;
   info[10] = (int64_t)h->bytes; info[11] = h->launches;
   info[12] = h->nprob;
   info[13] = h->kp.mpk;
@@ -1784,6 +1972,7 @@ int gm_info_ex(gm_handle h, int64_t* info, int count) {
   v[16] = h->l2_window ? (int64_t)h->window.num_bytes : 0;
   v[17] = h->kp.stage_cap;
   v[18] = h->kp.dep_mode;
+  v[19] = h->res ? 1 : 0;
   for (int i = 0; i < count && i < GM_INFO_EX_COUNT; ++i) info[i] = v[i];
   return GM_OK;
 }

@@ -26,12 +26,15 @@
 
 namespace gm {
 
+constexpr int kResThreads = 640;   // largest block of the resident entry points
+
 enum Phase : int {
   PH_LANCZOS = 1, PH_TRISOLVE = 2, PH_COEF = 4, PH_APPLY = 8,
   PH_UPDATE_FKPP = 16, PH_UPDATE_FHN = 32, PH_DEFLATE = 64,
   PH_APPLY_SET = 128,  // apply writes X = lift (fused solve) instead of X += lift
   PH_MPK = 256,        // compile-time only: entry points with matrix-powers Horner passes
-  PH_REORTH = 512      // compile-time only: entry points with Gram-Schmidt reorthogonalisation
+  PH_REORTH = 512,     // compile-time only: entry points with Gram-Schmidt reorthogonalisation
+  PH_RESIDENT = 1024   // compile-time only: entry points whose Lanczos phase keeps the problem on chip
 };
 
 struct KParams {
@@ -101,6 +104,18 @@ struct KParams {
   int reorth;
   double* hpart;    // [2][m + 8][R][G] per-block partial dots
   double* hblk;     // [G][m + 1][R] each block's totals
+  // Resident Lanczos phase (fab_resident.cuh): per SELL slot entry the column
+  // in block-local numbering (own slots, then the halo of halo_ptr/halo_rows),
+  // per slot whether another block references the row, the tagged words of
+  // exchanged rows [2][n][R] and of block partials [2][G][kRedStride], the
+  // offset of the state in dynamic shared memory and its capacities (entries, vector
+  // elements per right-hand side)
+  const unsigned short* res_col;
+  const unsigned char* res_exp;
+  ulonglong2* res_words;
+  ulonglong2* res_red;
+  ulonglong2* res_slice;     // mixed: sums of slices for other blocks' groups, [nslices][kRedStride]
+  int res_off, res_ent, res_vec;
   int* status;
   int* meff;        // [R]
   unsigned long long timeout_ns;
@@ -1606,6 +1621,12 @@ __device__ bool phase_deflate(const KParams& kp, const Ctx& c, int mode) {
   return true;
 }
 
+}  // namespace gm
+
+#include "fab_resident.cuh"
+
+namespace gm {
+
 // ------------------------------------------------------------------ kernel
 // Phase groups compiled as separate entry points.
 constexpr int KG_LANCZOS = PH_LANCZOS;
@@ -1642,7 +1663,7 @@ template <class Pol, int R, int PH>
 #ifndef GM_MINB1L2
 #define GM_MINB1L2 2   // one right-hand side, mixed, matrix held in the L2 window (PolMixedL2)
 #endif
-__global__ void __launch_bounds__(PH == KG_SOLVE ? kSolveThreads : GM_MAXT, (PH == KG_SOLVE ? 3 : R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
+__global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : PH == KG_SOLVE ? kSolveThreads : GM_MAXT, ((PH & PH_RESIDENT) ? 1 : PH == KG_SOLVE ? 3 : R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
                                             : (R == 1 ? ((PH & (PH_MPK | PH_REORTH)) ? GM_MINB1X
                                                                                      : (Pol::kL2 ? GM_MINB1L2 : GM_MINB1))
                                                       : GM_MINB))) fab_kernel(KParams kp) {
@@ -1660,7 +1681,11 @@ __global__ void __launch_bounds__(PH == KG_SOLVE ? kSolveThreads : GM_MAXT, (PH 
   };
   if ((PH & PH_LANCZOS) && (ph & PH_LANCZOS)) {
     if (!sep()) return;
-    if (!phase_lanczos<Pol, R, (PH & PH_MPK) != 0, (PH & PH_REORTH) != 0>(kp, c, g, ps, cs)) return;
+    if constexpr ((PH & PH_RESIDENT) != 0) {
+      if (!phase_lanczos_resident<Pol, R>(kp, c)) return;
+    } else {
+      if (!phase_lanczos<Pol, R, (PH & PH_MPK) != 0, (PH & PH_REORTH) != 0>(kp, c, g, ps, cs)) return;
+    }
   }
   if ((PH & PH_TRISOLVE) && (ph & PH_TRISOLVE)) {
     if (!sep()) return;

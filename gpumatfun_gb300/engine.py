@@ -401,7 +401,7 @@ class Engine:
         keys = ("n", "nrhs", "m", "d", "C", "k", "precision", "grid_blocks", "threads",
                 "sell_padded", "device_bytes", "launches", "problems", "matrix_powers",
                 "value_prefetch_bytes", "reorth", "l2_window_bytes", "col_stage_groups",
-                "neighbour_waits")
+                "neighbour_waits", "resident")
         v = (ct.c_int64 * len(keys))()
         self._check(self._lib.gm_info_ex(self._h, v, len(keys)))
         return dict(zip(keys, list(v)))

@@ -355,9 +355,11 @@ int gm_info(gm_handle h, int64_t* info16);
  * persisting access-policy window (0: no window, the matrix streams from
  * HBM on every pass), [17] column-index staging depth in 32-column groups
  * per stage (0: staging off), [18] 1 when passes wait on their neighbour
- * blocks only, 0 when every pass ends at a grid barrier.  Fills the first
+ * blocks only, 0 when every pass ends at a grid barrier, [19] 1 when the
+ * Lanczos phase keeps the problem on chip (small problems with every
+ * launch-shape option at its default).  Fills the first
  * min(count, GM_INFO_EX_COUNT) entries. */
-#define GM_INFO_EX_COUNT 19
+#define GM_INFO_EX_COUNT 20
 int gm_info_ex(gm_handle h, int64_t* info, int count);
 
 /* Effective Krylov dimension per (problem, RHS) after the last build (< m
