@@ -22,11 +22,11 @@
 // bounded condition number for CholQR) and is capped by max_degree.
 //
 // Layout: block vectors [n][32] row-major (one row of the block is 256
-// contiguous bytes), so lane j of a warp owns column j: the SpMM gathers
-// X[c][0..31] as one coalesced 256-byte row per stored entry, and every
+// contiguous bytes): the SpMM gathers X[c][0..31] as one coalesced 256-byte row
+// per stored entry, two columns per lane of half a warp, and every
 // 32 x 32 product (Gram matrices, X W) is a per-row multiply with the small
 // matrix in shared memory.  The matrix is CSR (int64 row pointer, int32
-// column indices, FP64 values), one warp per row.
+// column indices, FP64 values).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,41 +60,67 @@ int eig_fail(int code, const char* fmt, ...) {
   return code;
 }
 
-// Y_out = c1 (A X) + c2 X + c3 Y_prev, lane = column, one warp per row.
+// Y_out = c1 (A X) + c2 X + c3 Y_prev: half a warp per row, two neighbouring
+// columns per lane, so that a gathered row of X is one 256-byte access of 16
+// lanes and its index, value and address are formed once for two columns.
 // A row has few stored entries, so the kernel waits on the dependent chain
 // of memory accesses (row pointer, then column indices and values, then the
-// gathered rows of X).  The chain is shortened: the next row's pointers are
-// loaded while the current row is processed, and the epilogue's X and Y_prev
-// rows are loaded before the gathers.  Entries are taken 8 at a time, their
-// gathers all in flight before the products.
+// gathered rows of X); two rows per warp put twice the chains in flight.  The
+// next row's pointers are loaded while the current row is processed, and the
+// epilogue's X and Y_prev rows are loaded before the gathers.  Entries are
+// taken kChebU at a time, their gathers all in flight before the products.
+// Against one row per warp and one column per lane, on a 60k-node disk with
+// k = 20 (4,133 float-float and 869 FP64 steps of 32 columns): 214 -> 142 ms
+// for the whole iteration, 65 ms of it from k_jacobi; four entries at a time
+// 142, eight 139.
+constexpr int kChebU = 8;
+
+// Thousands of these kernels follow one another, each a few microseconds: they
+// are launched with programmatic stream serialization, so that a kernel's
+// blocks start while the last one drains, read their row pointers (the matrix
+// does not change) and wait here for the vectors.
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __global__ void k_cheb(long long n, const long long* __restrict__ rp, const int* __restrict__ ci,
-                       const double* __restrict__ va, const double* __restrict__ X,
-                       const double* __restrict__ Yp, double* __restrict__ Yo, double c1, double c2, double c3) {
-  const int lane = threadIdx.x & 31;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+                       const double* __restrict__ va, const double* X, const double* Yp, double* Yo, double c1,
+                       double c2, double c3) {
+  const int hl = threadIdx.x & 15;
+  const double2* X2 = reinterpret_cast<const double2*>(X) + hl;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 4;
+  long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  dependents_may_launch();
   long long b = r < n ? rp[r] : 0, e = r < n ? rp[r + 1] : 0;
+  wait_for_previous();
   for (; r < n; r += nw) {
     const long long rn = r + nw;
     const long long bn = rn < n ? rp[rn] : 0, en = rn < n ? rp[rn + 1] : 0;
-    const double xo = c2 != 0.0 ? X[r * P + lane] : 0.0;
-    const double yo = c3 != 0.0 ? Yp[r * P + lane] : 0.0;
-    double acc = 0.0;
-    for (long long t = b; t < e; t += 8) {
-      double av[8], xv[8];
+    const double2 z = make_double2(0.0, 0.0);
+    const double2 xo = c2 != 0.0 ? X2[r * (P / 2)] : z;
+    const double2 yo = c3 != 0.0 ? reinterpret_cast<const double2*>(Yp)[r * (P / 2) + hl] : z;
+    double2 acc = z;
+    const int* cp = ci + b;
+    const double* vp = va + b;
+    for (int t = (int)(e - b); t > 0; t -= kChebU, cp += kChebU, vp += kChebU) {
+      double av[kChebU];
+      double2 xv[kChebU];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+      for (int q = 0; q < kChebU; ++q) {
         av[q] = 0.0;
-        xv[q] = 0.0;
-        if (t + q < e) {
-          av[q] = __ldg(va + t + q);
-          xv[q] = __ldg(X + (long long)__ldg(ci + t + q) * P + lane);
+        xv[q] = z;
+        if (q < t) {
+          av[q] = __ldg(vp + q);
+          xv[q] = X2[(long long)__ldg(cp + q) * (P / 2)];
         }
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc = fma(av[q], xv[q], acc);
+      for (int q = 0; q < kChebU; ++q) {
+        acc.x = fma(av[q], xv[q].x, acc.x);
+        acc.y = fma(av[q], xv[q].y, acc.y);
+      }
     }
-    Yo[r * P + lane] = fma(c3, yo, fma(c2, xo, c1 * acc));
+    reinterpret_cast<double2*>(Yo)[r * (P / 2) + hl] =
+        make_double2(fma(c3, yo.x, fma(c2, xo.x, c1 * acc.x)), fma(c3, yo.y, fma(c2, xo.y, c1 * acc.y)));
     b = bn;
     e = en;
   }
@@ -107,46 +133,62 @@ __global__ void k_cheb(long long n, const long long* __restrict__ rp, const int*
 // rounding error in lo, renormalised once per row.  About 12 FP32
 // instructions per product instead of one FP64 FMA on GB300's narrow FP64
 // pipe.  Memory access order as in k_cheb.
-__global__ void k_cheb_ff(long long n, const long long* __restrict__ rp, const int* __restrict__ ci,
-                          const float* __restrict__ vhi, const float* __restrict__ vlo,
-                          const float2* __restrict__ X, const float2* __restrict__ Yp, float2* __restrict__ Yo,
-                          float2 c1, float2 c2, float2 c3) {
+__device__ __forceinline__ void cheb_ff_acc(float& hi, float& lo, float2 a, float xh, float xl) {
+  const gm::ff p = gm::two_prod(a.x, xh);
+  const float cross = fmaf(a.x, xl, a.y * xh);
+  const gm::ff s2 = gm::two_sum(hi, p.hi);
+  hi = s2.hi;
+  lo += s2.lo + (p.lo + cross);
+}
+__device__ __forceinline__ gm::ff cheb_ff_out(float hi, float lo, float xh, float xl, float yh, float yl, float2 c1,
+                                              float2 c2, float2 c3) {
   using gm::ff;
-  const int lane = threadIdx.x & 31;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  const float2 z = make_float2(0.f, 0.f);
-  long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  ff y = gm::ff_mul(gm::fast_two_sum(hi, lo), ff{c1.x, c1.y});
+  if (c2.x != 0.f) y = gm::ff_add(y, gm::ff_mul(ff{xh, xl}, ff{c2.x, c2.y}));
+  if (c3.x != 0.f) y = gm::ff_add(y, gm::ff_mul(ff{yh, yl}, ff{c3.x, c3.y}));
+  return y;
+}
+__global__ void k_cheb_ff(long long n, const long long* __restrict__ rp, const int* __restrict__ ci,
+                          const float* __restrict__ vhi, const float* __restrict__ vlo, const float2* X,
+                          const float2* Yp, float2* Yo, float2 c1, float2 c2, float2 c3) {
+  const int hl = threadIdx.x & 15;
+  const float4* X4 = reinterpret_cast<const float4*>(X) + hl;   // (hi, lo) of two columns
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 4;
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  dependents_may_launch();
   long long b = r < n ? rp[r] : 0, e = r < n ? rp[r + 1] : 0;
+  wait_for_previous();
   for (; r < n; r += nw) {
     const long long rn = r + nw;
     const long long bn = rn < n ? rp[rn] : 0, en = rn < n ? rp[rn + 1] : 0;
-    const float2 xo = c2.x != 0.f ? X[r * P + lane] : z;
-    const float2 yo = c3.x != 0.f ? Yp[r * P + lane] : z;
-    float ahi = 0.f, alo = 0.f;
-    for (long long t = b; t < e; t += 8) {
-      float2 av[8], xv[8];
+    const float4 xo = c2.x != 0.f ? X4[r * (P / 2)] : z;
+    const float4 yo = c3.x != 0.f ? reinterpret_cast<const float4*>(Yp)[r * (P / 2) + hl] : z;
+    float h0 = 0.f, l0 = 0.f, h1 = 0.f, l1 = 0.f;
+    const int* cp = ci + b;
+    const float* hp = vhi + b;
+    const float* lp = vlo + b;
+    for (int t = (int)(e - b); t > 0; t -= kChebU, cp += kChebU, hp += kChebU, lp += kChebU) {
+      float2 av[kChebU];
+      float4 xv[kChebU];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        av[q] = z;
+      for (int q = 0; q < kChebU; ++q) {
+        av[q] = make_float2(0.f, 0.f);
         xv[q] = z;
-        if (t + q < e) {
-          av[q] = make_float2(__ldg(vhi + t + q), __ldg(vlo + t + q));
-          xv[q] = __ldg(X + (long long)__ldg(ci + t + q) * P + lane);
+        if (q < t) {
+          av[q] = make_float2(__ldg(hp + q), __ldg(lp + q));
+          xv[q] = X4[(long long)__ldg(cp + q) * (P / 2)];
         }
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const ff p = gm::two_prod(av[q].x, xv[q].x);
-        const float cross = fmaf(av[q].x, xv[q].y, av[q].y * xv[q].x);
-        const ff s2 = gm::two_sum(ahi, p.hi);
-        ahi = s2.hi;
-        alo += s2.lo + (p.lo + cross);
+      for (int q = 0; q < kChebU; ++q) {
+        cheb_ff_acc(h0, l0, av[q], xv[q].x, xv[q].y);
+        cheb_ff_acc(h1, l1, av[q], xv[q].z, xv[q].w);
       }
     }
-    ff y = gm::ff_mul(gm::fast_two_sum(ahi, alo), ff{c1.x, c1.y});
-    if (c2.x != 0.f) y = gm::ff_add(y, gm::ff_mul(ff{xo.x, xo.y}, ff{c2.x, c2.y}));
-    if (c3.x != 0.f) y = gm::ff_add(y, gm::ff_mul(ff{yo.x, yo.y}, ff{c3.x, c3.y}));
-    Yo[r * P + lane] = make_float2(y.hi, y.lo);
+    const gm::ff a = cheb_ff_out(h0, l0, xo.x, xo.y, yo.x, yo.y, c1, c2, c3);
+    const gm::ff c = cheb_ff_out(h1, l1, xo.z, xo.w, yo.z, yo.w, c1, c2, c3);
+    reinterpret_cast<float4*>(Yo)[r * (P / 2) + hl] = make_float4(a.hi, a.lo, c.hi, c.lo);
     b = bn;
     e = en;
   }
@@ -188,12 +230,22 @@ __global__ void __launch_bounds__(1024) k_gram(long long n, long long rows_per_b
   partial[(long long)blockIdx.x * (P * P) + t] = acc;
 }
 
-// out[t] = sum over the G blocks of partial[b][t], in block order (deterministic).
+// out[t] = sum over the G blocks of partial[b][t], in block order
+// (deterministic); 16 loads ahead of the additions, a serial chain of 64 cycles
+// each (32 -> 10 us for 304 blocks).
 __global__ void k_gram_sum(const double* __restrict__ partial, int G, double* __restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P * P) return;
   double s = 0.0;
-  for (int b = 0; b < G; ++b) s += partial[(long long)b * (P * P) + t];
+  int b = 0;
+  for (; b + 16 <= G; b += 16) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = partial[(long long)(b + u) * (P * P) + t];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += v[u];
+  }
+  for (; b < G; ++b) s += partial[(long long)b * (P * P) + t];
   out[t] = s;
 }
 
@@ -243,120 +295,136 @@ __global__ void k_take_cols(long long n, int k, const double* __restrict__ X, do
   }
 }
 
-// One warp: G = L L^T (Cholesky, L lower), then M = L^{-T} (so that X M has
-// orthonormal columns).  status[0] = 1 when G is not numerically positive
-// definite (a pivot at or below 1e-14 of the largest diagonal entry).
-__global__ void k_chol_inv(const double* __restrict__ Gin, double* __restrict__ M, int* __restrict__ status) {
+// G = L L^T (Cholesky, L lower), then M = L^{-T} (so that X M has orthonormal
+// columns).  status[0] = 1 when G is not numerically positive definite (a pivot
+// at or below 1e-14 of the largest diagonal entry).
+// One block, warp i and lane j at entry (i, j): each of the 32 steps of the
+// factorisation and of the substitution is one update of every entry (one
+// warp did them entry by entry, 92 us).
+__global__ void __launch_bounds__(1024) k_chol_inv(const double* __restrict__ Gin, double* __restrict__ M,
+                                                   int* __restrict__ status) {
   __shared__ double L[P][P + 1];
   __shared__ double Li[P][P + 1];
   __shared__ int bad;
-  const int lane = threadIdx.x;
-  for (int i = 0; i < P; ++i) L[i][lane] = Gin[i * P + lane];
-  if (lane == 0) bad = 0;
-  __syncwarp();
+  const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
+  double a = Gin[threadIdx.x];
+  L[i][lane] = a;
+  if (threadIdx.x == 0) bad = 0;
+  __syncthreads();
   double dmax = 0.0;
-  for (int i = 0; i < P; ++i) dmax = fmax(dmax, L[i][i]);
+  for (int t = 0; t < P; ++t) dmax = fmax(dmax, L[t][t]);
+  __syncthreads();
   for (int k = 0; k < P; ++k) {
-    if (lane == 0) {
-      const double d = L[k][k];
-      if (!(d > 1e-14 * dmax)) bad = 1;
-      L[k][k] = sqrt(fmax(d, 1e-300));
+    if (i == k && lane == k) {
+      if (!(a > 1e-14 * dmax)) bad = 1;
+      a = sqrt(fmax(a, 1e-300));
+      L[k][k] = a;
     }
-    __syncwarp();
-    if (lane > k) L[lane][k] /= L[k][k];
-    __syncwarp();
-    for (int j = k + 1; j < P; ++j)
-      if (lane >= j) L[lane][j] -= L[lane][k] * L[j][k];
-    __syncwarp();
+    __syncthreads();
+    if (i > k && lane == k) {
+      a /= L[k][k];
+      L[i][k] = a;
+    }
+    __syncthreads();
+    if (i > k && lane > k && lane <= i) a -= L[i][k] * L[lane][k];
   }
-  // column `lane` of L^{-1} by forward substitution
-  for (int i = 0; i < P; ++i) {
-    double s = i == lane ? 1.0 : 0.0;
-    for (int t = 0; t < i; ++t) s -= L[i][t] * Li[t][lane];
-    Li[i][lane] = i >= lane ? s / L[i][i] : 0.0;
-    __syncwarp();
+  // L^{-1} by forward substitution, row t of all columns at once
+  double s = i == lane ? 1.0 : 0.0;
+  for (int t = 0; t < P; ++t) {
+    if (i == t) Li[t][lane] = t >= lane ? s / L[t][t] : 0.0;
+    __syncthreads();
+    if (i > t) s -= L[i][t] * Li[t][lane];
   }
-  // M[i][j] = (L^{-1})[j][i]
-  for (int i = 0; i < P; ++i) M[i * P + lane] = Li[lane][i];
-  if (lane == 0) status[0] = bad;
+  M[threadIdx.x] = Li[lane][i];   // M[i][j] = (L^{-1})[j][i]
+  if (threadIdx.x == 0) status[0] = bad;
 }
 
-// One warp: eigendecomposition of the symmetric 32 x 32 H by cyclic Jacobi
-// rotations (G. H. Golub, C. F. Van Loan, Matrix Computations, 4th ed.,
-// Algorithm 8.5.2 and 8.5.3), FP64.  theta ascending, W[i][j] = component i
-// of eigenvector j.
-__global__ void k_jacobi(const double* __restrict__ Hin, double* __restrict__ theta, double* __restrict__ W) {
+// Eigendecomposition of the symmetric 32 x 32 H by cyclic Jacobi rotations
+// (G. H. Golub, C. F. Van Loan, Matrix Computations, 4th ed., Algorithms 8.5.2
+// and 8.5.3), FP64.  theta ascending, W[i][j] = component i of eigenvector j.
+// The rotations of a sweep in cyclic order by rows, (0, 1), (0, 2), ..,
+// (30, 31), depend on each other only through a shared index, and the pairs
+// with p + q = t share none while every earlier rotation that touches p or q
+// has a smaller sum: a sweep is 61 steps of up to 16 rotations, the same
+// rotations up to rounding.  One block; warp i and lane j hold H(i, j) and
+// V(j, i), and every update is by rows through shared memory: H <- J^T H,
+// then J^T of its transpose, and the columns of V as rows.  A warp whose index
+// has no partner in the step skips its arithmetic (half of them on average).
+// What bounds it is FP64 issue: about 1,500 cycles for a step's angles and
+// 1,850 for its updates, where V's run while warp 0 forms the next angles.
+// (One warp, one rotation at a time: 6.6 ms a call.)
+__global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ Hin, double* __restrict__ theta,
+                                                 double* __restrict__ W) {
   __shared__ double H[P][P + 1];
-  __shared__ double V[P][P + 1];
-  __shared__ double cs[2];
-  __shared__ int order[P];
-  const int lane = threadIdx.x;
-  for (int i = 0; i < P; ++i) {
-    H[i][lane] = 0.5 * (Hin[i * P + lane] + Hin[lane * P + i]);
-    V[i][lane] = i == lane ? 1.0 : 0.0;
-  }
-  __syncwarp();
+  __shared__ double T[P][P + 1];
+  __shared__ double Vs[P][P + 1];
+  __shared__ double cc[2][P], ss[2][P];   // by step parity: x_i <- cc x_i + ss x_partner
+  __shared__ double red[2][P];
+  const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
+  const unsigned full = 0xffffffffu;
+  auto partner = [](int t, int k) { return t - k >= 0 && t - k < P ? t - k : k; };
+  double h = 0.5 * (Hin[i * P + lane] + Hin[lane * P + i]);
+  double v = i == lane ? 1.0 : 0.0;
+  H[i][lane] = h;
+  Vs[i][lane] = v;
+  __syncthreads();
   for (int sweep = 0; sweep < 30; ++sweep) {
-    double off = 0.0, tot = 0.0;
-    for (int i = 0; i < P; ++i) {
-      const double h = H[i][lane];
-      tot += h * h;
-      if (i != lane) off += h * h;
+    const double h2 = h * h;
+    const double off = gm::warp_sum(i == lane ? 0.0 : h2), tot = gm::warp_sum(h2);
+    if (lane == 0) {
+      red[0][i] = off;
+      red[1][i] = tot;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    }
-    if (off <= 1e-30 * tot) break;
-    for (int p = 0; p < P - 1; ++p)
-      for (int q = p + 1; q < P; ++q) {
-        if (lane == 0) {
-          const double apq = H[p][q];
-          double c = 1.0, s = 0.0;
+    __syncthreads();
+    if (gm::warp_sum(red[0][lane]) <= 1e-30 * gm::warp_sum(red[1][lane])) break;   // the same in every warp
+    const int last = 2 * P - 3;
+    for (int t = 1; t <= last + 1; ++t) {
+      const int cur = t & 1, old = cur ^ 1;
+      // angles of step t by warp 0; V of step t - 1 by the others, then by warp 0
+      if (i == 0 && t <= last) {
+        const int pj = partner(t, lane);
+        double c = 1.0, s = 0.0;
+        if (pj > lane) {
+          const double apq = H[lane][pj];
           if (apq != 0.0) {
-            const double tau = (H[q][q] - H[p][p]) / (2.0 * apq);
-            const double t = tau >= 0.0 ? 1.0 / (tau + sqrt(1.0 + tau * tau)) : -1.0 / (-tau + sqrt(1.0 + tau * tau));
-            c = 1.0 / sqrt(1.0 + t * t);
-            s = t * c;
+            const double tau = (H[pj][pj] - H[lane][lane]) / (2.0 * apq);
+            const double r = sqrt(1.0 + tau * tau);
+            const double tn = tau >= 0.0 ? 1.0 / (tau + r) : -1.0 / (-tau + r);
+            c = rsqrt(1.0 + tn * tn);
+            s = tn * c;
           }
-          cs[0] = c;
-          cs[1] = s;
         }
-        __syncwarp();
-        const double c = cs[0], s = cs[1];
-        if (s != 0.0) {
-          // H <- J^T H J and V <- V J, J the rotation in the (p, q) plane
-          double a = H[lane][p], b = H[lane][q];
-          H[lane][p] = c * a - s * b;
-          H[lane][q] = s * a + c * b;
-          __syncwarp();
-          a = H[p][lane];
-          b = H[q][lane];
-          H[p][lane] = c * a - s * b;
-          H[q][lane] = s * a + c * b;
-          a = V[lane][p];
-          b = V[lane][q];
-          V[lane][p] = c * a - s * b;
-          V[lane][q] = s * a + c * b;
-          __syncwarp();
-          if (lane == 0) H[p][q] = H[q][p] = 0.0;
-        }
-        __syncwarp();
+        const double co = __shfl_sync(full, c, pj), so = __shfl_sync(full, s, pj);
+        cc[cur][lane] = pj < lane ? co : c;
+        ss[cur][lane] = pj < lane ? so : -s;
       }
+      const int qi = partner(t - 1, i);
+      if (t > 1 && qi != i) v = cc[old][i] * v + ss[old][i] * Vs[qi][lane];
+      __syncthreads();
+      if (t > 1 && qi != i) Vs[i][lane] = v;
+      if (t > last) break;
+      const int pi = partner(t, i);
+      const double ci = cc[cur][i], si = ss[cur][i];
+      if (pi != i) h = ci * h + si * H[pi][lane];
+      T[i][lane] = h;
+      __syncthreads();
+      h = T[lane][i];
+      if (pi != i) {
+        h = ci * h + si * T[lane][pi];
+        if (lane == pi && si != 0.0) h = 0.0;
+      }
+      H[i][lane] = h;
+      __syncthreads();
+    }
   }
-  if (lane == 0) {
-    for (int i = 0; i < P; ++i) order[i] = i;
-    for (int i = 0; i < P; ++i)
-      for (int j = i + 1; j < P; ++j)
-        if (H[order[j]][order[j]] < H[order[i]][order[i]]) {
-          const int t = order[i];
-          order[i] = order[j];
-          order[j] = t;
-        }
-  }
-  __syncwarp();
-  theta[lane] = H[order[lane]][order[lane]];
-  for (int i = 0; i < P; ++i) W[i * P + lane] = V[i][order[lane]];
+  // ascending order: rank of each diagonal entry
+  __syncthreads();
+  const double mine = H[lane][lane];
+  int rank = 0;
+  for (int j = 0; j < P; ++j) rank += H[j][j] < mine || (H[j][j] == mine && j < lane);
+  if (i == 0) theta[rank] = mine;
+  rank = __shfl_sync(full, rank, i);
+  W[lane * P + rank] = v;
 }
 
 struct Solver {
@@ -390,10 +458,24 @@ struct Solver {
 
   unsigned grid_rows() const { return (unsigned)std::max(1, nsm * 8); }   // 256-thread blocks, a warp per row
 
+  // 256-thread blocks, overlapping the tail of the kernel before (see k_cheb)
+  template <class... Args>
+  static cudaError_t launch_overlapped(void (*kernel)(Args...), unsigned grid, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+  }
+
   cudaError_t spmm_axpby(const double* X, const double* Yp, double* Yo, double c1, double c2, double c3) {
-    k_cheb<<<grid64, 256>>>(n, rp, ci, va, X, Yp, Yo, c1, c2, c3);
     ++spmm;
-    return cudaGetLastError();
+    return launch_overlapped(k_cheb, grid64, n, (const long long*)rp, (const int*)ci, (const double*)va, X, Yp, Yo, c1,
+                             c2, c3);
   }
 
   static float2 to_ff(double v) {
@@ -402,16 +484,16 @@ struct Solver {
   }
 
   cudaError_t spmm_axpby_ff(const float2* X, const float2* Yp, float2* Yo, double c1, double c2, double c3) {
-    k_cheb_ff<<<grid_ff, 256>>>(n, rp, ci, vhi, vlo, X, Yp, Yo, to_ff(c1), to_ff(c2), to_ff(c3));
     ++spmm;
     ++spmm_ff;
-    return cudaGetLastError();
+    return launch_overlapped(k_cheb_ff, grid_ff, n, (const long long*)rp, (const int*)ci, (const float*)vhi,
+                             (const float*)vlo, X, Yp, Yo, to_ff(c1), to_ff(c2), to_ff(c3));
   }
 
   // small[0..1024) = Y^T Z
   cudaError_t gram(const double* Y, const double* Z) {
     k_gram<<<G, 1024>>>(n, rows_per_block, Y, Z, part);
-    k_gram_sum<<<(P * P + 255) / 256, 256>>>(part, G, small);
+    k_gram_sum<<<P, P>>>(part, G, small);
     return cudaGetLastError();
   }
 
@@ -420,7 +502,7 @@ struct Solver {
   int cholqr2(double* X, double* tmp) {
     for (int pass = 0; pass < 2; ++pass) {
       if (gram(X, X) != cudaSuccess) return -1;
-      k_chol_inv<<<1, 32>>>(small, small + P * P, status);
+      k_chol_inv<<<1, 1024>>>(small, small + P * P, status);
       int bad = 0;
       if (cudaMemcpy(&bad, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
       if (bad) return 1;
@@ -546,7 +628,7 @@ extern "C" int gm_deflation_pairs(int64_t n, const int64_t* rowptr, const int32_
   auto rayleigh_ritz = [&](double* Yb) -> int {
     if (S.spmm_axpby(Yb, nullptr, T, 1.0, 0.0, 0.0) != cudaSuccess) return -1;
     if (S.gram(Yb, T) != cudaSuccess) return -1;
-    k_jacobi<<<1, 32>>>(S.small, S.small + 2 * P * P, S.small + P * P);
+    k_jacobi<<<1, 1024>>>(S.small, S.small + 2 * P * P, S.small + P * P);
     k_rowmul<<<S.grid_rows(), 256>>>(n, Yb, S.small + P * P, X);
     k_rowmul<<<S.grid_rows(), 256>>>(n, T, S.small + P * P, AX);
     k_resid<<<ge, 256>>>(n, AX, X, S.small + 2 * P * P, T);
