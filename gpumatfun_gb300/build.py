@@ -16,7 +16,8 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "_lib"
 LIB = Path(os.environ["GPUMATFUN_LIB"]) if os.environ.get("GPUMATFUN_LIB") else LIBDIR / "libgpumatfun.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["engine.cu", "kern_fp64.cu", "kern_mixed.cu", "kern_mixed_l2.cu", "kern_resident.cu", "noalloc.cu", "eigs.cu"]
+SOURCES = ["engine.cu", "kern_fp64.cu", "kern_mixed.cu", "kern_mixed_l2.cu", "kern_resident.cu", "kern_dia.cu",
+           "noalloc.cu", "eigs.cu"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
 # Kernel shape overrides for tuning builds, e.g. "-DGM_MINB1=2 -DGM_CH1=4"
 # (GM_MINB1 / GM_MINB / GM_MINB4: minimum resident 512-thread blocks per SM

@@ -26,6 +26,7 @@ void* kernel_fp64(int R, int group);
 void* kernel_mixed(int R, int group);
 void* kernel_mixed_l2(int group);
 void* kernel_resident(bool fp64, int R, bool fused);
+void* kernel_dia(bool fp64, int R, int group, bool l2);
 }  // namespace gm
 
 namespace {
@@ -72,6 +73,10 @@ struct gm_engine {
   bool mpk_req = false;          // matrix-powers passes requested
   long long mpk_nmax = 0;        // largest own + halo rows of a block
   std::vector<int> sell_col_host;  // SELL column indices kept for the halo build
+  bool dia_req = false;          // look for diagonal slices
+  bool dia = false;              // most slices are diagonals (kern_dia.cu)
+  std::vector<std::pair<int, int>> dia_pads;   // (row, column) of their zero entries
+  size_t val_bytes = 0;          // the values' share of the matrix allocation
   bool res = false;              // the Lanczos phase keeps the problem on chip (fab_resident.cuh)
   size_t res_word_bytes = 0;     // its tagged words (one allocation)
   std::vector<double> roww;      // mixed engine: weights of the diagonal compensation (empty = ones)
@@ -234,6 +239,91 @@ void append_block(Csr& A, const Csr& B, long long row0) {
   A.val.insert(A.val.end(), B.val.begin(), B.val.end());
 }
 
+// Diagonal slices.  A full slice is one when the union of its rows' offsets
+// (column minus row) is no longer than its longest row and every entry a row
+// lacks would still fall inside its problem: the slice then stores the union,
+// with zeros, and its columns follow from the row.  The entries keep the rows'
+// (ascending) order, the diagonal first where diag_first asks for it, and the
+// slice its length, so neither the sums nor the partition change.
+struct DiaSlices {
+  static constexpr int kLen = 16;                      // offsets per pattern, at most
+  std::vector<int> off;                                // [pattern][kLen], problem after problem
+  std::vector<int> len;                                // [pattern]
+  std::vector<int> pat0;                               // [problem + 1] its first pattern
+  std::vector<short> pat;                              // [slice] within its problem, -1: ordinary
+  long long count = 0;
+};
+DiaSlices find_dia(const Csr& A, const std::vector<long long>& prow0, const std::vector<long long>& pslice0,
+                   bool diag_first) {
+  DiaSlices D;
+  const int np = (int)prow0.size() - 1;
+  D.pat.assign(pslice0[np], -1);
+  const int max_pat = gm::kDiaTable / DiaSlices::kLen;
+  D.pat0.assign(1, 0);
+  for (int p = 0; p < np; ++p) {
+    const int base = D.pat0[p];
+    int last = -1;
+    for (long long s = pslice0[p]; s < pslice0[p + 1]; ++s) {
+      const long long r0 = prow0[p] + 32 * (s - pslice0[p]);
+      if (r0 + 32 > prow0[p + 1]) continue;
+      int u[DiaSlices::kLen], nu = 0, longest = 0;
+      bool ok = true;
+      if (diag_first) u[nu++] = 0;
+      for (long long r = r0; r < r0 + 32 && ok; ++r) {
+        longest = std::max<int>(longest, (int)std::min<long long>(A.ptr[r + 1] - A.ptr[r], 1000));
+        if (A.ptr[r + 1] - A.ptr[r] == nu) {
+          // most rows have the offsets of the one before
+          const int* c = A.col.data() + A.ptr[r];
+          int q = 0;
+          while (q < nu && c[q] - (int)r == u[q]) ++q;
+          if (q == nu) continue;
+        }
+        int at = 0;
+        long long before = -1;
+        bool has_diag = false;
+        for (long long t = A.ptr[r]; t < A.ptr[r + 1] && ok; ++t) {
+          const int o = A.col[t] - (int)r;
+          ok = A.col[t] > before;
+          before = A.col[t];
+          has_diag = has_diag || o == 0;
+          while (at < nu && u[at] < o) ++at;
+          if (at < nu && u[at] == o) continue;
+          if (nu == DiaSlices::kLen) { ok = false; break; }
+          for (int q = nu; q > at; --q) u[q] = u[q - 1];
+          u[at] = o;
+          ++nu;
+        }
+        if (diag_first && !has_diag) ok = false;   // (its explicit zero diagonal comes first)
+      }
+      if (!ok || nu == 0 || nu > longest) continue;
+      // every offset of every row inside the problem
+      if (r0 + u[0] < prow0[p] || r0 + 31 + u[nu - 1] >= prow0[p + 1]) continue;
+      if (diag_first) {
+        int z = 0;
+        while (u[z] != 0) ++z;
+        for (; z > 0; --z) u[z] = u[z - 1];
+        u[0] = 0;
+      }
+      auto same = [&](int q) { return D.len[q] == nu && std::equal(u, u + nu, D.off.begin() + q * DiaSlices::kLen); };
+      int id = last >= 0 && same(last) ? last : -1;
+      for (int q = base; id < 0 && q < (int)D.len.size(); ++q)
+        if (same(q)) id = q;
+      if (id < 0) {
+        if ((int)D.len.size() - base == max_pat) continue;
+        id = (int)D.len.size();
+        D.len.push_back(nu);
+        D.off.insert(D.off.end(), u, u + nu);
+        D.off.resize((size_t)(id + 1) * DiaSlices::kLen, 0);
+      }
+      D.pat[s] = (short)(id - base);
+      last = id;
+      ++D.count;
+    }
+    D.pat0.push_back((int)D.len.size());
+  }
+  return D;
+}
+
 // SELL-32 over the block-diagonal matrix: every problem starts on a new
 // slice, so a slice never mixes problems (pad slots map to row -1).
 template <class VT>
@@ -245,6 +335,11 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   // (an explicit zero one where the matrix has none).
   const bool diag_first = sizeof(VT) == 4 && e->comp;
   const long long nrows_all = (long long)A.ptr.size() - 1;
+  // A 2^-e: a product with the power of two (the same rounding), where that is
+  // a normal number
+  const bool plain = std::abs(scale_exp) <= 1000;
+  const double factor = plain ? std::ldexp(1.0, -scale_exp) : 0.0;
+  auto scaled = [&](double v) { return plain ? v * factor : std::ldexp(v, -scale_exp); };
   std::vector<long long> dpos;
   if (diag_first) {
     dpos.assign(nrows_all, -1);
@@ -260,6 +355,13 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   for (int p = 0; p < np; ++p) pslice0[p + 1] = pslice0[p] + (prow0[p + 1] - prow0[p] + 31) / 32;
   const long long nsl = pslice0[np];
   const bool sorted = sigma > 1;
+  // (three slices in four: below that the ordinary kernels' column stages serve
+  // the rest better)
+  DiaSlices D;
+  if (e->dia_req && !sorted) {
+    D = find_dia(A, prow0, pslice0, diag_first);
+    e->dia = 4 * D.count >= 3 * nsl;
+  }
   rows.assign(nsl * 32, -1);
   for (int p = 0; p < np; ++p) {
     const long long n_p = prow0[p + 1] - prow0[p];
@@ -281,6 +383,7 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
       const long long r = rows[s * 32 + l];
       if (r >= 0) L = std::max(L, row_len(r));
     }
+    if (L > 65535) e->dia = false;   // (16 bits hold a slice's length there)
     off[s + 1] = off[s] + 32 * L;
   }
   const long long padded = off[nsl];
@@ -289,8 +392,33 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   std::vector<VT> val(padded);
   std::vector<int> c2s;
   if (e->keep_map) c2s.assign(A.ptr.back(), 0);
+  int prob = 0;
   for (long long s = 0; s < nsl; ++s) {
     const long long L = (off[s + 1] - off[s]) / 32;
+    if (e->dia && D.pat[s] >= 0) {
+      while (s >= pslice0[prob + 1]) ++prob;
+      const int* u = D.off.data() + (D.pat0[prob] + D.pat[s]) * DiaSlices::kLen;
+      for (int l = 0; l < 32; ++l) {
+        const long long r = rows[s * 32 + l];
+        // the row's entries in ascending order; diag_first puts offset 0 first
+        long long t = A.ptr[r];
+        const long long te = A.ptr[r + 1];
+        for (long long jj = 0; jj < L; ++jj) {
+          const long long dst = off[s] + jj * 32 + l, c = r + u[jj];
+          long long at = -1;
+          if (diag_first && jj == 0) {
+            if (dpos[r] >= 0) at = te > t ? t + dpos[r] : -1;
+          } else {
+            if (diag_first && t < te && A.col[t] == r) ++t;
+            if (t < te && A.col[t] == c) at = t++;
+          }
+          col[dst] = (int)c;
+          val[dst] = at >= 0 ? (VT)scaled(A.val[at]) : (VT)0;
+          if (at < 0 && c != r) e->dia_pads.emplace_back((int)r, (int)c);
+        }
+      }
+      continue;
+    }
     for (int l = 0; l < 32; ++l) {
       const long long r = rows[s * 32 + l];
       const long long len = r >= 0 ? row_len(r) : 0;
@@ -312,7 +440,7 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
           }
           if (e->keep_map) c2s[A.ptr[r] + t] = (int)dst;
           col[dst] = A.col[A.ptr[r] + t];
-          val[dst] = (VT)std::ldexp(A.val[A.ptr[r] + t], -scale_exp);
+          val[dst] = (VT)scaled(A.val[A.ptr[r] + t]);
         } else {
           col[dst] = r >= 0 ? (int)r : 0;
           val[dst] = (VT)0;
@@ -323,7 +451,7 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   long long* d_off;
   int rc;
   if ((rc = dupload(e, &d_off, off.data(), off.size()))) return rc;
-  if (np == 1 && !sorted) e->sell_col_host = col;
+  if (np == 1 && !sorted && (e->mpk_req || nsl <= 16LL * e->nsm)) e->sell_col_host = col;
   // Diagonal compensation of the FP32-stored matrix: row r gets the extra
   // diagonal term c_r = sum_t (a_t 2^-e - fl32(a_t 2^-e)) w_col(t) / w_r, so
   // that the stored operator maps w exactly as A does.  The small eigenvalues
@@ -343,7 +471,7 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
         if (e->keep_map) r2s[r] = (int)(s * 32 + l);
         double corr = 0.0;
         for (long long t = A.ptr[r]; t < A.ptr[r + 1]; ++t) {
-          const double exact = std::ldexp(A.val[t], -scale_exp);
+          const double exact = scaled(A.val[t]);
           const double err = exact - (double)(float)exact;
           corr += ones ? err : err * e->roww[A.col[t]];
         }
@@ -373,6 +501,25 @@ int upload_sell(gm_engine* e, const Csr& A, int sigma, int scale_exp, const std:
   }
   e->mat_base = d_mat;
   e->mat_bytes = mbytes;
+  e->val_bytes = vbytes;
+  if (e->dia) {
+    std::vector<int2> meta(nsl);
+    for (long long s = 0; s < nsl; ++s)
+      meta[s] = make_int2((int)(off[s] / 32), (int)((unsigned)((off[s + 1] - off[s]) / 32) | ((unsigned)(unsigned short)D.pat[s] << 16)));
+    std::vector<int> shift(np);
+    for (int p = 0; p < np; ++p) shift[p] = (int)(32 * pslice0[p] - prow0[p]);
+    int2* d_meta;
+    int *d_po, *d_p0, *d_shift;
+    if ((rc = dupload(e, &d_meta, meta.data(), meta.size()))) return rc;
+    if ((rc = dupload(e, &d_po, D.off.data(), D.off.size()))) return rc;
+    if ((rc = dupload(e, &d_shift, shift.data(), shift.size()))) return rc;
+    if ((rc = dupload(e, &d_p0, D.pat0.data(), D.pat0.size()))) return rc;
+    e->kp.dia_pat0 = d_p0;
+    e->kp.dia_meta = d_meta;
+    e->kp.dia_off = d_po;
+    e->kp.dia_shift = d_shift;
+    e->kp.dia_len = DiaSlices::kLen;
+  }
   if (e->keep_map && (rc = dupload(e, &e->csr2sell, c2s.data(), c2s.size()))) return rc;
   if (e->keep_map && (rc = dupload(e, &e->csr_ptr, A.ptr.data(), A.ptr.size()))) return rc;
   e->kp.slice_off = d_off;
@@ -570,6 +717,17 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
           }
         }
       }
+  // a diagonal slice's zero entries are read too (times zero): their owners'
+  // rows must have been written
+  for (const auto& rc2 : e->dia_pads) {
+    const int q = owner[rc2.first], o = owner[rc2.second];
+    if (o != q) {
+      adj[(size_t)q * G + o] = 1;
+      adj[(size_t)o * G + q] = 1;
+    }
+  }
+  e->dia_pads.clear();
+  e->dia_pads.shrink_to_fit();
   // Matrix-powers passes: per block the halo rows (referenced by its rows,
   // owned elsewhere), local column indices, and waits over two hops.
   const bool mpk = e->mpk_req && !e->res && !e->sell_col_host.empty();
@@ -1020,6 +1178,11 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     }
     e->scale_exp = mx > 0.0 ? (int)std::floor(std::log2(mx)) : 0;
   }
+  // Diagonal slices: not where the stored entries must keep their CSR places
+  // (keep_entry_map, matrix powers), an explicit request for column stages, or
+  // problems small enough for the resident phase.
+  e->dia_req = !e->keep_map && !e->mpk_req && a->col_staging != 2 && a->sell_sigma <= 1 &&
+               (ntot + 31) / 32 > 16LL * e->nsm;
   std::vector<long long> slot_rows, slice_off, pslice0;
   rc = e->prec == GM_FP64 ? upload_sell<double>(e, csr, a->sell_sigma, 0, prow0, slot_rows, slice_off, pslice0)
                           : upload_sell<float>(e, csr, a->sell_sigma, e->scale_exp, prow0, slot_rows, slice_off, pslice0);
@@ -1073,8 +1236,8 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   // (whose level-between vector shares the dynamic shared memory) stage
   // whenever the slices fit a stage.
   const bool stage_l2 = e->prec == GM_FP64 && !e->mpk_req;
-  const bool staging = a->col_staging == 2 ||
-                       (a->col_staging == 0 && (!use_window || a->val_prefetch == 1 || stage_l2));
+  const bool staging = !e->dia && (a->col_staging == 2 ||
+                       (a->col_staging == 0 && (!use_window || a->val_prefetch == 1 || stage_l2)));
   // Resident Lanczos phase: one block per SM with at most one slice per warp,
   // the problem on chip between passes.  It is the engine's own choice of a
   // launch shape: taken only where every launch-shape option is at its
@@ -1108,7 +1271,7 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   const size_t stage_smem = stage_bytes(e->threads);
   e->kp.stage_cap = stage_cap;
   e->kp.pf_vals = 0;
-  if (stage_cap > 0 && a->val_prefetch != 2) {
+  if ((stage_cap > 0 || e->dia) && a->val_prefetch != 2) {
     if (a->val_prefetch == 1 || !use_window) e->kp.pf_vals = e->prec == GM_FP64 ? 8 : 4;
   }
   // Grid: blocks_per_sm x SMs, capped by co-residency of each phase-group
@@ -1154,6 +1317,18 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   e->G = (int)Gmax;
   // blocks per problem and the slice partition (sets e->G to the blocks used)
   if ((rc = build_partition(e, csr, slot_rows, slice_off, pslice0, prow0, plan))) return rc;
+  if (e->dia) {
+    // the same grid and threads as the ordinary entry points
+    for (int g : {KGRP_LANCZOS, KGRP_APPLY, KGRP_LANCZOS_RO}) {
+      // (an apply without a polynomial has no SpMV)
+      if ((g == KGRP_LANCZOS_RO && a->reorth == 0) || (g == KGRP_APPLY && e->d == 0)) continue;
+      void* k = gm::kernel_dia(e->prec == GM_FP64, e->R, g, l2k);
+      int nb = 0;
+      GM_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, e->Tk[g], e->smem[g]));
+      if ((long long)nb * e->nsm < e->Gk[g]) return fail(e, GM_ERR_UNSUPPORTED, "diagonal-slice kernel group %d: grid does not fit", g);
+      e->kfn[g] = k;
+    }
+  }
   // The shifted solves and the coefficients take few warps, each bound by FP64
   // issue: spread over the SMs, without grid barriers.
   e->Gk[KGRP_SOLVE] = 2 * e->nsm;
@@ -1193,7 +1368,8 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     // handle with a window is deleted (window_acquire / window_release).
     int max_window = 0;
     GM_CUDA(e, cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, e->dev));
-    const size_t win = std::min<size_t>(e->mat_bytes, (size_t)max_window);
+    // (diagonal slices read the values only, which come first)
+    const size_t win = std::min<size_t>(e->dia ? e->val_bytes : e->mat_bytes, (size_t)max_window);
     GM_CUDA(e, window_acquire(e->dev, win));
     e->window.base_ptr = e->mat_base;
     e->window.num_bytes = win;

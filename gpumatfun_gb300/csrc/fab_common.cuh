@@ -115,6 +115,7 @@ struct PolFP64 {
   using ST = double;   // scalar used in per-element operations
   static constexpr bool kMixed = false;
   static constexpr bool kL2 = false;
+  static constexpr bool kDia = false;
   __device__ static __forceinline__ AT zero() { return 0.0; }
   __device__ static __forceinline__ ST scalar(double s) { return s; }
   __device__ static __forceinline__ AT acc(AT a, VT v, double x) { return fma(v, x, a); }
@@ -142,6 +143,7 @@ struct PolMixed {
   using ST = ff;
   static constexpr bool kMixed = true;
   static constexpr bool kL2 = false;
+  static constexpr bool kDia = false;
   __device__ static __forceinline__ AT zero() { return {0.f, 0.f}; }
   __device__ static __forceinline__ ST scalar(double s) { return ff_from_double(s); }
   // SpMV row accumulation: hi gathers the exactly-split products (two_sum),
@@ -213,6 +215,13 @@ struct PolMixed {
 // FP64 engine, which spills little at 40 registers, measured slower with two
 // blocks on the same L2-held disk (21.2 vs 19.2 ms) and has no such variant.
 struct PolMixedL2 : PolMixed { static constexpr bool kL2 = true; };
+
+// The same arithmetic for matrices whose slices are mostly diagonals: every
+// row of such a slice references the same offsets from itself (the stencil of
+// a regular grid), so the kernels need no column indices and no stages.
+struct PolFP64Dia : PolFP64 { static constexpr bool kDia = true; };
+struct PolMixedDia : PolMixed { static constexpr bool kDia = true; };
+struct PolMixedL2Dia : PolMixedL2 { static constexpr bool kDia = true; };
 
 __device__ __forceinline__ double h_to_d(double h) { return h; }
 __device__ __forceinline__ double h_to_d(float2 h) { return (double)h.x + (double)h.y; }

@@ -90,6 +90,15 @@ struct KParams {
   const long long* prob_row0; // [nprob+1] first row of each problem
   int stage_cap;              // >0: stage each slice's column indices in shared memory by TMA
   int pf_vals;                // >0: L2 bulk prefetch of the next slice's values (bytes per value)
+  // Diagonal slices: per slice (first entry / 32, entries per row | pattern <<
+  // 16; pattern -1: an ordinary slice), the patterns' offsets from the row
+  // [pattern][dia_len] by problem (dia_pat0), and per problem 32 * its first
+  // slice - its first row
+  const int2* dia_meta;
+  const int* dia_off;
+  const int* dia_pat0;
+  const int* dia_shift;
+  int dia_len;
   // Two Horner levels per pass (matrix powers): per block, the rows its rows
   // reference outside its own range (halo), the SELL column indices in block-
   // local numbering (own rows first, then the halo), and the offset of the
@@ -292,6 +301,62 @@ __device__ __forceinline__ void row_entries1(const int* __restrict__ cp, const t
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], a, xv[r]);
   }
+}
+
+// Entries of a diagonal slice row: the row's vector entries at fixed offsets,
+// so index and gather are not a chain of two loads and neighbouring lanes read
+// neighbouring entries.  DiaWidth entries are loaded before their products: six
+// with one right-hand side (160^3 mixed 86.4 us per step with three, 84.8 with
+// two, 82.1 with six), else as many as fit the registers without more spills.
+// Against column indices, per step: 160^3 mixed 96.6 -> 82.1 us, 500^2 mixed
+// with four right-hand sides 62 -> 38, 24 grids up to 512^2 67 -> 61, 117^3
+// FP64 61.3 -> 57.3 (bound by FP64 issue), 700^2 FP64 28.4 -> 27.3.  The
+// entries keep the row's order, with a zero value where a row lacks an offset
+// that its slice has.
+template <class Pol, int R>
+struct DiaWidth {
+  static constexpr int value = R == 1 ? 6 : (R == 4 && !Pol::kMixed ? 1 : 2);
+};
+template <class Pol, int R, class XT>
+__device__ __forceinline__ void row_dia(const int* of, const typename Pol::VT* __restrict__ vp, int len,
+                                        const XT* __restrict__ xr, float dl, typename Pol::AT (&acc)[R]) {
+  constexpr int U = DiaWidth<Pol, R>::value;
+  if constexpr (Pol::kMixed) {
+    // entry 0 is the diagonal (see spmv_slot); dl is zero without compensation
+    XT xv[R];
+    VecIO<R>::ld(xr + of[0] * R, xv);
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], dl, xv[r]);
+  }
+  int jj = 0;
+  for (; jj + U <= len; jj += U) {
+    typename Pol::VT a[U];
+    XT xv[U][R];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      a[u] = ld_val(vp + (jj + u) * 32);
+      VecIO<R>::ld(xr + of[jj + u] * R, xv[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], a[u], xv[u][r]);
+  }
+  for (; U > 1 && jj < len; ++jj) {
+    XT xv[R];
+    const typename Pol::VT a = ld_val(vp + jj * 32);
+    VecIO<R>::ld(xr + of[jj] * R, xv);
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], a, xv[r]);
+  }
+}
+
+// The offsets of the patterns of the block's problem and its row shift, in
+// shared memory.
+constexpr int kDiaTable = 512;
+__device__ __forceinline__ int* dia_table() {
+  __shared__ int s_dia[kDiaTable + 1];
+  return s_dia;
 }
 
 template <class Pol, int R, class XT>
@@ -526,7 +591,7 @@ struct ColStage {
 };
 
 // One SpMV pass over the block's slices: z = A x for the slice rows, then
-// epi(s, z) for the row epilogue.  rowpf: the [n][R] storage-precision
+// epi(row, z) for the row epilogue (row -1: padding).  rowpf: the [n][R] storage-precision
 // vector the epilogue reads at the slice rows and that the gathers of x do
 // not bring into cache (prefetched one slice ahead with the values when the
 // matrix streams from HBM), or null.
@@ -540,6 +605,47 @@ __device__ __forceinline__ bool spmv_pass(const KParams& kp, const Ctx& c, ColSt
   constexpr unsigned kRowB = R <= 2 ? (unsigned)(R * sizeof(typename Pol::BT)) : 0u;
   const long long sb = kp.blk_slice[c.b()], se = kp.blk_slice[c.b() + 1];
   long long s = sb + c.warp();
+  if constexpr (Pol::kDia) {
+    // no stages: the slice's place and pattern one slice ahead, and with a
+    // matrix streamed from HBM the bulk prefetch of its values and of the
+    // epilogue's rows
+    using VT = typename Pol::VT;
+    const int* const tab = dia_table();
+    int2 mt = s < se ? __ldg(kp.dia_meta + s) : make_int2(0, 0);
+    if (wait && !wait->before_next(kp)) return false;
+    for (; s < se; s += c.nw()) {
+      const long long sn = s + c.nw();
+      const int2 mn = sn < se ? __ldg(kp.dia_meta + sn) : make_int2(0, 0);
+      if (kp.pf_vals && sn < se && c.lane() == 0) {
+        tma_bulk_prefetch_l2(static_cast<const unsigned char*>(kp.val) + (long long)mn.x * 32 * kp.pf_vals,
+                             (unsigned)kp.pf_vals * 32u * (unsigned)(mn.y & 0xffff));
+        if (kRowB > 0 && rowpf && tab[kDiaTable] == 0 && (mn.y >> 16) >= 0)
+          tma_bulk_prefetch_l2(reinterpret_cast<const unsigned char*>(rowpf) + sn * 32 * kRowB, 32u * kRowB);
+      }
+      const int len = mt.y & 0xffff, pat = mt.y >> 16;
+      const VT* vp = reinterpret_cast<const VT*>(kp.val) + (long long)mt.x * 32 + c.lane();
+      float dl = 0.f;
+      if constexpr (Pol::kMixed) {
+        if (kp.dlo) dl = __ldg(kp.dlo + s * 32 + c.lane());
+      }
+      AT z[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) z[r] = Pol::zero();
+      long long row;
+      if (pat >= 0) {
+        row = s * 32 + c.lane() - tab[kDiaTable];
+        row_dia<Pol, R, XT>(tab + pat * kp.dia_len, vp, len, x + row * R, dl, z);
+      } else {
+        row = slot_row(kp, s, c.lane());
+        row_entries1<Pol, R, XT, false>(kp.col + (long long)mt.x * 32 + c.lane(), vp, len, x, dl, z);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) z[r] = Pol::norm(z[r]);
+      epi(row, z);
+      mt = mn;
+    }
+    return true;
+  }
   if (kRowB > 0 && c.lane() == 0) *ColStage::row_pf_slot() = rowpf;
   if (s < se) cs.issue<kRowB>(kp, 0, s, c.lane());
   // the ordering wait on the previous pass comes after the first column copy
@@ -557,7 +663,7 @@ __device__ __forceinline__ bool spmv_pass(const KParams& kp, const Ctx& c, ColSt
     spmv_slot<Pol, R, XT>(kp, s, c.lane(), x, z, scol);
 #pragma unroll
     for (int r = 0; r < R; ++r) z[r] = Pol::norm(z[r]);
-    epi(s, z);
+    epi(slot_row(kp, s, c.lane()), z);
     cs.release();
   }
   return true;
@@ -619,9 +725,8 @@ __device__ __forceinline__ bool horner_pair(const KParams& kp, const Ctx& c, Col
   const long long rb0 = sb * 32;
   const long long nown = (se * 32 < kp.n ? se * 32 : kp.n) - rb0;
   // level 1, own rows (the usual pass, results to shared memory)
-  const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long s, AT (&z)[R]) {
-    const long long row = s * 32 + c.lane();
-    if (row >= kp.n) return;
+  const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long row, AT (&z)[R]) {
+    if (row < 0) return;
     BT sv[R];
     VecIO<R>::ld(w + row * R, sv);
     HT u[R];
@@ -926,8 +1031,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
 #pragma unroll
     for (int r = 0; r < R; ++r) apa[r] = Pol::zero();
     if (d == 0) {
-      spmv_pass<Pol, R, BT>(kp, c, cs, src, [&](long long s, AT (&z)[R]) {
-        const long long row = slot_row(kp, s, c.lane());
+      spmv_pass<Pol, R, BT>(kp, c, cs, src, [&](long long row, AT (&z)[R]) {
         if (row < 0) return;
         BT sv[R], v[R];
         VecIO<R>::ld(src + row * R, sv);
@@ -951,8 +1055,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
     } else {
       // Horner pass 1: u = gamma_1 v_j + A (gamma_0 v_j); stores v_j
       {
-        spmv_pass<Pol, R, BT>(kp, c, cs, src, [&](long long s, AT (&z)[R]) {
-          const long long row = slot_row(kp, s, c.lane());
+        spmv_pass<Pol, R, BT>(kp, c, cs, src, [&](long long row, AT (&z)[R]) {
           if (row < 0) return;
           BT sv[R], v[R];
           VecIO<R>::ld(src + row * R, sv);
@@ -980,8 +1083,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
         }
         for (; h <= d; ++h, ++k) {
           HT* hout = (k & 1) ? H1 : H0;
-          const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, (k & 1) ? H0 : H1, [&](long long s, AT (&z)[R]) {
-            const long long row = slot_row(kp, s, c.lane());
+          const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, (k & 1) ? H0 : H1, [&](long long row, AT (&z)[R]) {
             if (row < 0) return;
             BT sv[R];
             VecIO<R>::ld(src + row * R, sv);
@@ -999,8 +1101,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
         for (int h = 2; h <= d; ++h) {
           const HT* hin_h = (h & 1) ? H0 : H1;
           HT* hout = (h & 1) ? H1 : H0;
-          const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin_h, [&](long long s, AT (&z)[R]) {
-            const long long row = slot_row(kp, s, c.lane());
+          const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin_h, [&](long long row, AT (&z)[R]) {
             if (row < 0) return;
             BT sv[R];
             VecIO<R>::ld(src + row * R, sv);
@@ -1015,8 +1116,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
         hin = (d & 1) ? H1 : H0;
       }
       // final pass: w = A u - beta_j v_{j-1}
-      const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long s, AT (&z)[R]) {
-        const long long row = slot_row(kp, s, c.lane());
+      const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long row, AT (&z)[R]) {
         if (row < 0) return;
         BT sv[R];
         VecIO<R>::ld(src + row * R, sv);
@@ -1388,7 +1488,12 @@ __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool 
   constexpr int IC = 3;
   const long long sb = kp.blk_slice[c.b()], se = kp.blk_slice[c.b() + 1];
   for (long long s = sb + c.warp(); s < se; s += c.nw()) {
-    const long long i = slot_row(kp, s, c.lane());
+    long long i;
+    if constexpr (Pol::kDia) {
+      i = (__ldg(kp.dia_meta + s).y >> 16) >= 0 ? s * 32 + c.lane() - dia_table()[kDiaTable] : slot_row(kp, s, c.lane());
+    } else {
+      i = slot_row(kp, s, c.lane());
+    }
     if (i < 0) continue;
     for (int i0 = 0; i0 < d1; i0 += IC) {
       AT acc[IC][R];
@@ -1447,8 +1552,7 @@ __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool 
     const HT* hin = h == 1 ? P : ((h & 1) ? H0 : H1);
     HT* hout = (h & 1) ? H1 : H0;
     const HT* Ph = P + (long long)h * n * R;
-    const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long s, AT (&z)[R]) {
-      const long long row = slot_row(kp, s, c.lane());
+    const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin, [&](long long row, AT (&z)[R]) {
       if (row < 0) return;
       HT p[R];
       VecIO<R>::ld(Ph + row * R, p);
@@ -1673,7 +1777,15 @@ __global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : PH == KG_SO
   const Grp g(kp, c);
   PassSync ps{kp.dep_mode, g.p, 0u};
   ColStage cs;
-  if (PH & (PH_LANCZOS | PH_APPLY)) cs.init(kp, c);
+  if constexpr (Pol::kDia) {
+    int* const tab = dia_table();
+    const int p0 = kp.dia_pat0[g.p], pn = kp.dia_pat0[g.p + 1] - p0;
+    for (int t = c.tid(); t < pn * kp.dia_len; t += c.nt()) tab[t] = kp.dia_off[p0 * kp.dia_len + t];
+    if (c.tid() == 0) tab[kDiaTable] = kp.dia_shift[g.p];
+    __syncthreads();
+  } else if (PH & (PH_LANCZOS | PH_APPLY)) {
+    cs.init(kp, c);
+  }
   bool first = true;
   auto sep = [&]() -> bool {
     if (first) { first = false; return true; }
