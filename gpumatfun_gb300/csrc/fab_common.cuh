@@ -289,9 +289,19 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
   return t;
 }
 
+// Grid barriers poll with relaxed loads and fence once at the end: an acquire
+// per poll drops the SM's L1 lines each time, the other resident blocks' too
+// (24 grids, four right-hand sides 58.8 -> 56.0 us per step).  The neighbour
+// waits, mostly over at the first read, poll with acquire loads: there the
+// fence costs more (500k disk, degree 8, 119.6 against 116.0 us per step).
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
@@ -315,36 +325,41 @@ struct GridBar {
   unsigned nblocks;
   unsigned long long timeout_ns;
 
+  // One thread's arrival for its block, and its wait for the others (the
+  // block's stores are ordered before it by a block barrier).  A block that
+  // records an error leaves and never arrives again, so the others find the
+  // status in their next wait: no read of it after a wait that succeeded (a
+  // round trip per barrier).
+  __device__ bool arrive_and_wait() const {
+    if (nblocks <= 1) return true;
+    bool ok = true;
+    unsigned long long* c64 = count;
+    __threadfence();
+    const unsigned long long old = atomicAdd(c64, 1ull);
+    const unsigned long long target = (old / nblocks + 1ull) * nblocks;
+    if (old + 1ull != target) {
+      unsigned long long t0 = global_timer_ns();
+      unsigned spins = 0;
+      while (ld_relaxed_u64(c64) < target) {
+        if ((++spins & 3u) == 0u) {
+          if ((spins & 31u) == 0u && *(volatile int*)status != 0) { ok = false; break; }
+          if (global_timer_ns() - t0 > timeout_ns) {
+            atomicCAS(status, 0, (int)ST_TIMEOUT);
+            ok = false;
+            break;
+          }
+        }
+        __nanosleep(32);
+      }
+    }
+    __threadfence();
+    return ok;
+  }
+
   __device__ bool sync() const {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int ok = 1;
-      if (nblocks > 1) {
-        unsigned long long* c64 = count;
-        __threadfence();
-        const unsigned long long old = atomicAdd(c64, 1ull);
-        const unsigned long long target = (old / nblocks + 1ull) * nblocks;
-        if (old + 1ull != target) {
-          unsigned long long t0 = global_timer_ns();
-          unsigned spins = 0;
-          while (ld_acquire_u64(c64) < target) {
-            if ((++spins & 3u) == 0u) {
-              if ((spins & 31u) == 0u && *(volatile int*)status != 0) { ok = 0; break; }
-              if (global_timer_ns() - t0 > timeout_ns) {
-                atomicCAS(status, 0, (int)ST_TIMEOUT);
-                ok = 0;
-                break;
-              }
-            }
-            __nanosleep(32);
-          }
-        }
-        __threadfence();
-      }
-      if (*(volatile int*)status != 0) ok = 0;
-      s_ok = ok;
-    }
+    if (threadIdx.x == 0) s_ok = arrive_and_wait();
     __syncthreads();
     return s_ok != 0;
   }
@@ -370,10 +385,9 @@ struct DepSync {
 
   __device__ void publish(unsigned pass) const {
     __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release_u64(prog + blockIdx.x, base + pass);
-    }
+    // (the release store orders the block's stores by itself; a fence ahead of
+    // it cost the disks' steps 4 to 7 %)
+    if (threadIdx.x == 0) st_release_u64(prog + blockIdx.x, base + pass);
   }
 
   __device__ bool wait(unsigned pass) const {
@@ -402,7 +416,7 @@ struct DepSync {
         }
       }
       ok = __all_sync(0xffffffffu, ok);
-      if (threadIdx.x == 0) s_ok = ok && (*(volatile int*)status == 0);
+      if (threadIdx.x == 0) s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;

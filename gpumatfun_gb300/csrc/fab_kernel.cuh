@@ -806,27 +806,177 @@ __device__ __forceinline__ bool horner_pair(const KParams& kp, const Ctx& c, Col
 #endif
 template <class Pol, int R>
 struct LanczosScalars {
-  double beta[R], rbeta[R], rbp[R], alpha[R], tot[R];
+  double beta[R], rbeta[R], rbp[R], alpha[R], bound[R];
   int broken[R];
   typename Pol::ST sc[R], rb[R], bj[R], al[R];
   typename Pol::ST gr[GM_MAX_DEG + 1][R];   // gamma_h rbeta_j of the current step
-  int all_broken;
+  double gam[GM_MAX_DEG + 1];
 };
 
-// Every block sums the G per-block partials (layout [N][G]) in one fixed
-// order into dst (shared memory); deterministic and identical in all blocks.
-// One warp per quantity: a lane's additions are a serial chain of FP64 issue
-// slots, 2.4 us for four right-hand sides in one warp.
-template <int N>
-__device__ __forceinline__ void grid_total_smem(const double* partials, int stride, int count, double* dst) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = warp; j < N; j += nw) {
-    double t = 0.0;
-    for (int b = lane; b < count; b += 32) t += partials[(long long)j * stride + b];
-    t = warp_sum(t);
-    if (lane == 0) dst[j] = t;
+// Where a problem's alpha, beta and m_eff go; lead: the one thread that writes.
+struct LanczosOut {
+  double* aab;
+  int* meff;
+  bool lead;
+};
+
+// The scalars of right-hand side r, each function by one full warp: different
+// lanes form the products and conversions at once, since an FP64 instruction
+// takes 64 cycles of issue for one lane as for 32.
+//
+// alpha_j = w^T v_j = rbeta_j (w^T w_j); pass B subtracts alpha_j rbeta_j w_j.
+template <class Pol, int R>
+__device__ __forceinline__ void step_alpha(LanczosScalars<Pol, R>& sh, int r, double tot) {
+  const double al = tot * sh.rbeta[r];
+  const typename Pol::ST q = Pol::scalar(al * sh.rbeta[r]);
+  if ((threadIdx.x & 31) == 0) {
+    sh.alpha[r] = al;
+    sh.al[r] = q;
+  }
+}
+// Off the critical path, after step_alpha: alpha's store and the bound of the
+// breakdown test, bd_tol (|alpha_j| + beta_j).
+template <class Pol, int R>
+__device__ __forceinline__ void step_bound(LanczosScalars<Pol, R>& sh, const KParams& kp, const LanczosOut& out, int r,
+                                           int j) {
+  const double al = sh.alpha[r];
+  if (out.lead) out.aab[j + (long long)(kp.m + 1) * r] = sh.broken[r] ? 0.0 : al;
+  if ((threadIdx.x & 31) == 0) {
+    sh.bound[r] = kp.bd_tol * (fabs(al) + (j > 0 ? sh.beta[r] : 0.0));
+    if (out.lead && !(al == al)) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
+  }
+  __syncwarp();
+}
+// From tot = beta^2: the end of step j, or beta_0 = ||U_r|| for j < 0.
+template <class Pol, int R>
+__device__ __forceinline__ void step_beta(LanczosScalars<Pol, R>& sh, const KParams& kp, const LanczosOut& out, int r,
+                                          double tot, int j) {
+  const int lane = threadIdx.x & 31, m = kp.m, d = kp.d;
+  const int hi = __double2hiint(tot);
+  const bool normal = hi >= 0x00100000 && hi < 0x7ff00000;
+  double rb, bn;
+  if (normal && !Pol::kMixed) {
+    // 1/sqrt(tot), and sqrt(tot) with its residual corrected (the mixed engine
+    // keeps the bits of the square root and the division)
+    rb = rsqrt(tot);
+    const double b0 = tot * rb;
+    bn = fma(fma(-b0, b0, tot), 0.5 * rb, b0);
+  } else {
+    bn = sqrt(tot);
+    rb = 1.0 / bn;
+  }
+  const int was = j < 0 ? 0 : sh.broken[r];
+  int broken = was;
+  if (j < 0) {
+    broken = !normal && !(bn > 0.0);
+  } else if (!broken && j + 1 < m) {
+    // positive numbers compare like their bits
+    const bool down = normal ? __double_as_longlong(bn) <= __double_as_longlong(sh.bound[r]) : !(bn > sh.bound[r]);
+    if (down) {
+      broken = 1;
+      if (out.lead) out.meff[r] = j + 1;
+    }
+  }
+  const double rb_old = j < 0 ? 0.0 : sh.rbeta[r];
+  if (out.lead) {
+    out.aab[(j + 1) + (long long)(m + 1) * (R + r)] = was ? 0.0 : bn;
+    if (j < 0) out.meff[r] = broken ? 0 : m;
+    if (!normal && (!(bn == bn) || isinf(bn))) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
+  }
+  const double be = broken && j >= 0 ? 0.0 : bn;
+  if (broken) rb = 0.0;
+  __syncwarp();   // every lane has read the old values
+  if (lane == 0) {
+    sh.broken[r] = broken;
+    sh.rbp[r] = rb_old;
+    sh.beta[r] = be;
+    sh.rbeta[r] = rb;
+  }
+  // lane 0: rbeta, lane 1: beta_j rbeta_{j-1}, lane 2 + h: gamma_h rbeta
+  const double f = lane == 0 ? 1.0 : lane == 1 ? rb_old : lane - 2 <= d ? sh.gam[lane - 2] : 0.0;
+  const typename Pol::ST q = Pol::scalar((lane == 1 ? be : rb) * f);
+  if (lane == 0) sh.rb[r] = q;
+  if (lane == 1) sh.bj[r] = q;
+  if (lane == 2) sh.sc[r] = q;
+  if (lane > 2 && lane - 2 <= d) sh.gr[lane - 2][r] = q;
+  for (int h = 30 + lane; h <= d; h += 32) sh.gr[h][r] = Pol::scalar(sh.gam[h] * rb);
+}
+
+// Sum of p[r] over the problem's blocks, then fin(r, total) with one full warp
+// per right-hand side; also the problem's grid barrier.  The tree is fixed:
+// the 32 lanes of a warp, the warps of a block, then each lane's blocks in
+// order and the lanes.  With one or two right-hand sides the lanes' trees run
+// from shared memory, eight lanes to a warp's sum (six FP64 additions in a
+// quarter of the warps instead of five in all of them: with 48 warps per SM
+// 2.2 us of issue), and so do the totals, whose loads are then one round trip.
+// Ends with a block barrier; false when a wait failed.
+template <int R>
+struct ReduceBuf {
+  static constexpr bool kStage = R <= 2;
+  static constexpr int kCap = 512;
+  double v[kStage ? R : 1][kStage ? kCap : 1];
+  double w[32][R];
+  int ok;
+};
+template <int R, class Fin>
+__device__ __forceinline__ bool reduce_blocks(ReduceBuf<R>& buf, const KParams& kp, const Ctx& c, const Grp& g,
+                                              double (&p)[R], double* part, Fin&& fin) {
+  constexpr bool kStage = ReduceBuf<R>::kStage;
+  constexpr int kCap = ReduceBuf<R>::kCap;
+  auto& s_v = buf.v;
+  auto& s_w = buf.w;
+  const int lane = c.lane(), warp = c.warp(), nw = c.nw(), G = kp.G;
+  if constexpr (kStage) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) s_v[r][c.tid()] = p[r];
+    __syncthreads();
+    for (int item = c.tid() >> 3; item < ((R * nw + 3) & ~3); item += c.nt() >> 3) {
+      const int it = item < R * nw ? item : R * nw - 1;   // whole warps for the shuffles
+      const int r = it / nw, w = it - r * nw, i = lane & 7;
+      const double* v = s_v[r] + w * 32 + i;
+      double t = (v[0] + v[16]) + (v[8] + v[24]);
+      t += __shfl_xor_sync(0xffffffffu, t, 4);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      if (i == 0) s_w[w][r] = t;
+    }
+  } else {
+    const double s = warp_sum_packed<R>(p);
+    if ((lane & (32 / R - 1)) == 0) s_w[warp][packed_index<R>(lane)] = s;
   }
   __syncthreads();
+  if (warp == 0) {
+    double t[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) t[r] = lane < nw ? s_w[lane][r] : 0.0;
+    const double q = warp_sum_packed<R>(t);
+    if ((lane & (32 / R - 1)) == 0) part[(long long)packed_index<R>(lane) * G + c.b()] = q;
+    __syncwarp();
+    if (lane == 0) buf.ok = g.bar(kp).arrive_and_wait();
+  }
+  __syncthreads();
+  if (!buf.ok) return false;
+  const double* pg = part + g.gb;
+  const bool staged = kStage && g.Gp <= kCap;
+  if constexpr (kStage) {
+    if (staged) {
+      for (int b = c.tid(); b < g.Gp; b += c.nt())
+#pragma unroll
+        for (int r = 0; r < R; ++r) s_v[r][b] = pg[(long long)r * G + b];
+      __syncthreads();
+    }
+  }
+  for (int r = warp; r < R; r += nw) {
+    double t = 0.0;
+    const double* v = pg + (long long)r * G;
+    if constexpr (kStage) {
+      if (staged) v = s_v[r];
+    }
+    for (int b = lane; b < g.Gp; b += 32) t += v[b];
+    fin(r, warp_sum(t));
+  }
+  __syncthreads();
+  return true;
 }
 
 // The per-block Gram-Schmidt coefficient x as the policy's scalar: FP64, or
@@ -871,16 +1021,33 @@ __device__ bool reorth_step(const KParams& kp, const Ctx& c, const Grp& g, int j
       for (int u = 0; u < TT; ++u)
 #pragma unroll
         for (int r = 0; r < R; ++r) acc[u][r] = Pol::zero();
-      for (long long i = g.gt(kp); i < g.r1(kp); i += g.tt()) {
-        HT wh[R];
-        VecIO<R>::ld(Hw + i * R, wh);
+      if (t0 + TT <= j + 1) {
+        // a whole tile: its loads before its products (with a guard per vector
+        // the compiler ordered them either way, 117^3 275 or 337 us per step
+        // from one build to the next)
+        for (long long i = g.gt(kp); i < g.r1(kp); i += g.tt()) {
+          HT wh[R];
+          VecIO<R>::ld(Hw + i * R, wh);
+          BT v[TT][R];
 #pragma unroll
-        for (int u = 0; u < TT; ++u) {
-          if (t0 + u <= j) {
-            BT v[R];
-            VecIO<R>::ld(V + ((long long)(t0 + u) * n + i) * R, v);
+          for (int u = 0; u < TT; ++u) VecIO<R>::ld(V + ((long long)(t0 + u) * n + i) * R, v[u]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) acc[u][r] = Pol::dot(acc[u][r], h_load_at<Pol>(wh[r]), v[r]);
+          for (int u = 0; u < TT; ++u)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[u][r] = Pol::dot(acc[u][r], h_load_at<Pol>(wh[r]), v[u][r]);
+        }
+      } else {
+        for (long long i = g.gt(kp); i < g.r1(kp); i += g.tt()) {
+          HT wh[R];
+          VecIO<R>::ld(Hw + i * R, wh);
+#pragma unroll
+          for (int u = 0; u < TT; ++u) {
+            if (t0 + u <= j) {
+              BT v[R];
+              VecIO<R>::ld(V + ((long long)(t0 + u) * n + i) * R, v);
+#pragma unroll
+              for (int r = 0; r < R; ++r) acc[u][r] = Pol::dot(acc[u][r], h_load_at<Pol>(wh[r]), v[r]);
+            }
           }
         }
       }
@@ -959,8 +1126,8 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
   using AT = typename Pol::AT;
   const long long n = kp.n;
   const int m = kp.m, d = kp.d, G = kp.G;
-  double* const aab = kp.aabb + (long long)(m + 1) * 2 * R * g.p;   // this problem's aabb
-  int* const meff = kp.meff + (long long)R * g.p;
+  const LanczosOut out{kp.aabb + (long long)(m + 1) * 2 * R * g.p, kp.meff + (long long)R * g.p,
+                       g.bl == 0 && c.lane() == 0};   // this problem's
   const double* const gam = kp.gamma + (long long)(d + 1) * g.p;
   BT* V = reinterpret_cast<BT*>(kp.V);
   BT* const W0 = reinterpret_cast<BT*>(kp.W0);
@@ -970,6 +1137,7 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
   double* part_a = kp.part;
   double* part_b = kp.part + (long long)R * G;
   __shared__ LanczosScalars<Pol, R> sh;
+  __shared__ ReduceBuf<R> buf;
 
   // prologue: W1 = U (storage precision), beta_0 = ||U_r||
   {
@@ -984,24 +1152,10 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
       for (int r = 0; r < R; ++r) { bp[r] = fma(u[r], u[r], bp[r]); wb[r] = (BT)u[r]; }
       VecIO<R>::st(W1 + i * R, wb);
     }
-    block_sum_store<R>(bp, part_b + c.b(), G);
+    if (c.tid() <= d) sh.gam[c.tid()] = gam[c.tid()];   // (read after reduce_blocks' barriers)
+    if (!reduce_blocks<R>(buf, kp, c, g, bp, part_b, [&](int r, double t) { step_beta<Pol, R>(sh, kp, out, r, t, -1); }))
+      return false;
   }
-  if (!group_bar(kp, g.p).sync()) return false;
-  grid_total_smem<R>(part_b + g.gb, G, g.Gp, sh.tot);
-  if (c.tid() == 0) {
-    for (int r = 0; r < R; ++r) {
-      sh.beta[r] = sqrt(sh.tot[r]);
-      sh.broken[r] = !(sh.beta[r] > 0.0);
-      sh.rbeta[r] = sh.broken[r] ? 0.0 : 1.0 / sh.beta[r];
-      sh.rbp[r] = 0.0;
-      if (g.bl == 0) {
-        aab[(long long)(m + 1) * (R + r)] = sh.beta[r];
-        meff[r] = sh.broken[r] ? 0 : m;
-        if (!(sh.tot[r] == sh.tot[r]) || isinf(sh.tot[r])) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
-      }
-    }
-  }
-  __syncthreads();
   // Inside the recurrence the Lanczos vector is v_j = rbeta_j w_j, formed
   // from the stored work vector w_j (src) in the accumulator precision in
   // every pass, so the polynomial's terms all act on the same vector: its
@@ -1018,15 +1172,6 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
     // rounds once to storage (rounding before the subtraction would make the
     // storage error relative to |w| instead of to beta_{j+1} << |w|).
     HT* Hw = (d & 1) ? H0 : H1;
-    if (c.tid() == 0) {
-      for (int r = 0; r < R; ++r) {
-        sh.sc[r] = Pol::scalar(sh.rbeta[r] * gam[0]);
-        sh.rb[r] = Pol::scalar(sh.rbeta[r]);
-        sh.bj[r] = Pol::scalar(sh.beta[r] * sh.rbp[r]);
-        for (int h = 1; h <= d; ++h) sh.gr[h][r] = Pol::scalar(gam[h] * sh.rbeta[r]);
-      }
-    }
-    __syncthreads();
     AT apa[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) apa[r] = Pol::zero();
@@ -1140,19 +1285,10 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
       double ap[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) ap[r] = Pol::to_d(apa[r]);
-      block_sum_store<R>(ap, part_a + c.b(), G);
+      ps.done(kp);
+      if (!reduce_blocks<R>(buf, kp, c, g, ap, part_a, [&](int r, double t) { step_alpha<Pol, R>(sh, r, t); })) return false;
+      for (int r = c.warp(); r < R; r += c.nw()) step_bound<Pol, R>(sh, kp, out, r, j);
     }
-    ps.done(kp);
-    if (!group_bar(kp, g.p).sync()) return false;
-    grid_total_smem<R>(part_a + g.gb, G, g.Gp, sh.alpha);
-    if (c.tid() == 0) {
-      // alpha_j = w^T v_j = rbeta_j (w^T w_j); pass B subtracts alpha_j rbeta_j w_j
-      for (int r = 0; r < R; ++r) {
-        sh.alpha[r] *= sh.rbeta[r];
-        sh.al[r] = Pol::scalar(sh.alpha[r] * sh.rbeta[r]);
-      }
-    }
-    __syncthreads();
     // pass B: w -= alpha_j v_j; beta_{j+1} = ||w||  (after the optional
     // Gram-Schmidt against V_0..V_j)
     {
@@ -1214,35 +1350,14 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
       double bp[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) bp[r] = Pol::to_d(bpa[r]);
-      block_sum_store<R>(bp, part_b + c.b(), G);
+      if (!reduce_blocks<R>(buf, kp, c, g, bp, part_b, [&](int r, double t) { step_beta<Pol, R>(sh, kp, out, r, t, j); }))
+        return false;
     }
-    if (!group_bar(kp, g.p).sync()) return false;
-    grid_total_smem<R>(part_b + g.gb, G, g.Gp, sh.tot);
-    if (c.tid() == 0) {
-      int all = 1;
-      for (int r = 0; r < R; ++r) {
-        const double bn = sqrt(sh.tot[r]);
-        const double al = sh.alpha[r];
-        if (g.bl == 0) {
-          aab[j + (long long)(m + 1) * r] = sh.broken[r] ? 0.0 : al;
-          aab[(j + 1) + (long long)(m + 1) * (R + r)] = sh.broken[r] ? 0.0 : bn;
-          if (!(bn == bn) || isinf(bn) || !(al == al)) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
-        }
-        const double scale = fabs(al) + (j > 0 ? sh.beta[r] : 0.0);
-        if (!sh.broken[r] && j + 1 < m && !(bn > kp.bd_tol * scale)) {
-          sh.broken[r] = 1;
-          if (g.bl == 0) meff[r] = j + 1;
-        }
-        sh.rbp[r] = sh.rbeta[r];
-        sh.beta[r] = sh.broken[r] ? 0.0 : bn;
-        sh.rbeta[r] = sh.broken[r] ? 0.0 : 1.0 / bn;
-        all = all && sh.broken[r];
-      }
-      sh.all_broken = all;
-    }
-    __syncthreads();
     src = Wout;
-    if (sh.all_broken) break;
+    bool all = true;
+#pragma unroll
+    for (int r = 0; r < R; ++r) all = all && sh.broken[r];
+    if (all) break;
   }
   return true;
 }

@@ -391,68 +391,8 @@ __device__ bool phase_lanczos_resident(const KParams& kp, const Ctx& c) {
   Resident<Pol, R> rs;
   rs.init(kp);
   BT* const V = reinterpret_cast<BT*>(kp.V);
-  const bool lead = c.b() == 0 && c.lane() == 0;
-
-  // Step scalars of right-hand side r from tot = beta^2, by one full warp
-  // (j < 0: beta_0 = ||U_r||; else the end of step j).  Breakdown: beta_{j+1}
-  // at most bd_tol (|alpha_j| + beta_j), the bound prepared by pre_beta.
-  const double gl = c.lane() >= 2 && c.lane() - 2 <= d ? kp.gamma[c.lane() - 2] : 1.0;
-  auto pre_beta = [&](int r, int j) {
-    const double al = sh.alpha[r];
-    if (lead) kp.aabb[j + (long long)(m + 1) * r] = sh.broken[r] ? 0.0 : al;
-    if (c.lane() == 0) {
-      sh.tot[r] = kp.bd_tol * (fabs(al) + (j > 0 ? sh.beta[r] : 0.0));
-      if (lead && !(al == al)) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
-    }
-    __syncwarp();
-  };
-  auto set_beta = [&](int r, double tot, int j) {
-    const int hi = __double2hiint(tot);
-    const bool normal = hi >= 0x00100000 && hi < 0x7ff00000;
-    double rb, bn;
-    if (normal && !Pol::kMixed) {
-      // 1/sqrt(tot), and sqrt(tot) with its residual corrected
-      rb = rsqrt(tot);
-      const double b0 = tot * rb;
-      bn = fma(fma(-b0, b0, tot), 0.5 * rb, b0);
-    } else {
-      bn = sqrt(tot);
-      rb = 1.0 / bn;
-    }
-    int broken = j < 0 ? 0 : sh.broken[r];
-    if (j < 0) {
-      broken = !normal && !(bn > 0.0);
-    } else if (!broken && j + 1 < m) {
-      // positive numbers compare like their bits
-      const bool down = normal ? __double_as_longlong(bn) <= __double_as_longlong(sh.tot[r]) : !(bn > sh.tot[r]);
-      if (down) {
-        broken = 1;
-        if (lead) kp.meff[r] = j + 1;
-      }
-    }
-    const double rb_old = j < 0 ? 0.0 : sh.rbeta[r];
-    if (lead) {
-      kp.aabb[(j + 1) + (long long)(m + 1) * (R + r)] = j >= 0 && (sh.broken[r]) ? 0.0 : bn;
-      if (j < 0) kp.meff[r] = broken ? 0 : m;
-      if (!normal && (!(bn == bn) || isinf(bn))) atomicCAS(kp.status, 0, (int)ST_NONFINITE);
-    }
-    const double be = broken && j >= 0 ? 0.0 : bn;
-    if (broken) rb = 0.0;
-    __syncwarp();   // every lane has read the old values
-    if (c.lane() == 0) {
-      sh.broken[r] = broken;
-      sh.rbp[r] = rb_old;
-      sh.beta[r] = be;
-      sh.rbeta[r] = rb;
-    }
-    // lane 0: rbeta, lane 1: beta_j rbeta_{j-1}, lane 2 + h: gamma_h rbeta
-    const typename Pol::ST q = Pol::scalar((c.lane() == 1 ? be : rb) * (c.lane() == 1 ? rb_old : gl));
-    if (c.lane() == 0) sh.rb[r] = q;
-    if (c.lane() == 1) sh.bj[r] = q;
-    if (c.lane() == 2) sh.sc[r] = q;
-    if (c.lane() > 2 && c.lane() - 2 <= d) sh.gr[c.lane() - 2][r] = q;
-    for (int h = 30 + c.lane(); h <= d; h += 32) sh.gr[h][r] = Pol::scalar(kp.gamma[h] * rb);
-  };
+  const LanczosOut out{kp.aabb, kp.meff, c.b() == 0 && c.lane() == 0};
+  if (c.tid() <= d) sh.gam[c.tid()] = kp.gamma[c.tid()];
   auto read_halo = [&]() -> bool {
     const int w0 = c.nw() > R ? R : 0;   // the warps that do not reduce, or all
     if (c.warp() < w0) return true;
@@ -469,7 +409,7 @@ __device__ bool phase_lanczos_resident(const KParams& kp, const Ctx& c) {
     for (int r = 0; r < R; ++r) { sv[r] = (BT)u[r]; p[r] = u[r] * u[r]; }
     rs.post(kp, sv);
     if (!rs.reduce(kp, c, p, 1, rs.base + 1, [](int) {},
-                   [&](int r, double t) { set_beta(r, t, -1); }, read_halo))
+                   [&](int r, double t) { step_beta<Pol, R>(sh, kp, out, r, t, -1); }, read_halo))
       return false;
   }
   for (int j = 0; j < m; ++j) {
@@ -519,14 +459,8 @@ __device__ bool phase_lanczos_resident(const KParams& kp, const Ctx& c) {
         }
       }
     }
-    if (!rs.reduce(kp, c, p, 0, rs.base + 2 + 2 * (unsigned long long)j, [](int) {}, [&](int r, double t) {
-          // alpha_j = w^T v_j = rbeta_j (w^T w_j); w_{j+1} = w - alpha_j rbeta_j w_j
-          if (c.lane() == 0) {
-            const double al = t * sh.rbeta[r];
-            sh.alpha[r] = al;
-            sh.al[r] = Pol::scalar(al * sh.rbeta[r]);
-          }
-        }, []() { return true; }))
+    if (!rs.reduce(kp, c, p, 0, rs.base + 2 + 2 * (unsigned long long)j, [](int) {},
+                   [&](int r, double t) { step_alpha<Pol, R>(sh, r, t); }, []() { return true; }))
       return false;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -536,8 +470,8 @@ __device__ bool phase_lanczos_resident(const KParams& kp, const Ctx& c) {
       p[r] = rs.row >= 0 ? Pol::dot_self(Pol::zero(), x) : Pol::zero();
     }
     rs.post(kp, sv);
-    if (!rs.reduce(kp, c, p, 1, rs.base + 3 + 2 * (unsigned long long)j, [&](int r) { pre_beta(r, j); },
-                   [&](int r, double t) { set_beta(r, t, j); }, read_halo))
+    if (!rs.reduce(kp, c, p, 1, rs.base + 3 + 2 * (unsigned long long)j, [&](int r) { step_bound<Pol, R>(sh, kp, out, r, j); },
+                   [&](int r, double t) { step_beta<Pol, R>(sh, kp, out, r, t, j); }, read_halo))
       return false;
     bool all = true;
 #pragma unroll
