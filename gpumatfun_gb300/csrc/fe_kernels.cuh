@@ -75,8 +75,11 @@ __device__ __forceinline__ ff ff_madd(ff acc, float ah, float al, float bh, floa
   return fast_two_sum(s.hi, e);
 }
 
+constexpr int kLiftShifts = 8;      // shifts per block of k_fe_lift_ff
+constexpr int kLiftThreads = 128;   // at its 163 registers, three blocks per SM (256 threads: one)
+
 template <class BT>
-__global__ void __launch_bounds__(256) k_fe_lift_ff(long long n, int m, int C, const BT* __restrict__ Vb,
+__global__ void __launch_bounds__(kLiftThreads) k_fe_lift_ff(long long n, int m, int C, const BT* __restrict__ Vb,
                                                     const BT* __restrict__ Vg, int vstride,
                                                     const double2* __restrict__ yb, const double2* __restrict__ yg,
                                                     double2* __restrict__ Rout, double2* __restrict__ Sout,
@@ -84,16 +87,19 @@ __global__ void __launch_bounds__(256) k_fe_lift_ff(long long n, int m, int C, c
   // Zb[i][j] = sum_q Vb(q, i) yb'[j][q], Zg[i][j] = sum_q Vg(q, i) yg[j][q];
   // V element (q, i) of a side at V[(q n + i) vstride] (the b and g bases are
   // columns of one interleaved basis, or two separate bases).  One row per
-  // thread; shifts in chunks of JC, coefficients in tiles of QT Krylov
-  // vectors held split in shared memory.
-  constexpr int JC = 8, QT = 128;
+  // thread and one chunk of JC shifts per blockIdx.y, coefficients in tiles of
+  // QT Krylov vectors held split in shared memory.  (All chunks in one block,
+  // one after another, left a 40k-node mesh with eight warps per SM: 1,326 us
+  // against 851.)
+  constexpr int JC = kLiftShifts, QT = 128;
   __shared__ float4 sy4[2 * JC * QT];  // [side][jj][q]: (re hi, re lo, im hi, im lo)
   const int mb = min(*meff_b, m), mg = min(*meff_g, m);
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {   // block-uniform
     const long long i = i0 + threadIdx.x;
     const bool act = i < n;
-    for (int j0 = 0; j0 < C; j0 += JC) {
+    {
+      const int j0 = (int)blockIdx.y * JC;
       ff rr[JC], ri[JC], sr[JC], si[JC];
 #pragma unroll
       for (int jj = 0; jj < JC; ++jj) rr[jj] = ri[jj] = sr[jj] = si[jj] = ff{0.f, 0.f};
