@@ -1212,7 +1212,13 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     GM_CUDA(e, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, e->dev));
     const bool fits_limit = mp > 0 && mw > 0 && e->mat_bytes <= (size_t)std::min(mp, mw);
     const double vec_bytes = (double)ntot * e->R * (2.0 * 8.0 + (e->prec == GM_FP64 ? 8.0 : 4.0));
-    const bool fits_l2 = (double)e->mat_bytes + vec_bytes <= 0.9 * (double)l2;
+    // FP64 disks, per step with and without the window (degree 8, one
+    // right-hand side): 600k nodes 119 / 128 us, 800k (86 MB with its vectors)
+    // 156 / 162, 1M (108 MB) 207 / 196; four right-hand sides 300k (64 MB) 218 /
+    // 219, 500k (90 MB) 349 / 344.  The mixed engine's line stays where its
+    // choice of kernels, and with it the order of its sums, has been.
+    const double share = e->prec == GM_FP64 ? 0.69 : 0.9;
+    const bool fits_l2 = (double)e->mat_bytes + vec_bytes <= share * (double)l2;
     use_window = fits_limit && (a->l2_window == 2 || fits_l2);
   }
   // Column staging: per warp two stages of stage_cap * 32 column indices
