@@ -50,10 +50,10 @@ struct gm_engine {
   int scale_exp = 0;             // mixed engine: A stored as A * 2^-scale_exp
   unsigned long long epoch = 0;  // launch counter (progress-flag epochs)
   double dep_avg = 0.0;          // mean neighbour-list length per block
-  int Gk[8] = {};                // grid size per phase group (co-residency bound)
-  int Tk[8] = {};                // threads per block per phase group
-  void* kfn[8] = {};
-  size_t smem[8] = {};           // dynamic shared memory per phase group
+  int Gk[9] = {};                // grid size per phase group (co-residency bound)
+  int Tk[9] = {};                // threads per block per phase group
+  void* kfn[9] = {};
+  size_t smem[9] = {};           // dynamic shared memory per phase group
   std::vector<DevBuf> bufs;
   size_t bytes = 0;
   KParams kp{};
@@ -859,9 +859,9 @@ int build_partition(gm_engine* e, const Csr& A, const std::vector<long long>& ro
 }
 
 // Entry points (kern_*.cu): one phase group each; the resident Lanczos phase
-// also with the rest of a solve.
+// also with the rest of a solve; the apply's lift (k_lift) by itself.
 enum { KGRP_LANCZOS = 0, KGRP_SOLVE = 1, KGRP_APPLY = 2, KGRP_DEFLATE = 3, KGRP_LANCZOS_MPK = 4, KGRP_LANCZOS_RO = 5,
-       KGRP_LANCZOS_RES = 6, KGRP_FUSED_RES = 7, KGRP_N = 8 };
+       KGRP_LANCZOS_RES = 6, KGRP_FUSED_RES = 7, KGRP_LIFT = 8, KGRP_N = 9 };
 
 // The dynamic shared memory limit is an attribute of the kernel function,
 // shared by every handle of the process (per device): only ever raise it, so
@@ -919,7 +919,7 @@ void window_release(int dev) {
 // right-hand side then runs the SpMV groups compiled for two resident blocks
 // per SM (gm::PolMixedL2, no register spills).
 void* pick_kernel(int prec, int R, int group, bool l2) {
-  if (group >= KGRP_LANCZOS_RES) return gm::kernel_resident(prec == GM_FP64, R, group == KGRP_FUSED_RES);
+  if (group == KGRP_LANCZOS_RES || group == KGRP_FUSED_RES) return gm::kernel_resident(prec == GM_FP64, R, group == KGRP_FUSED_RES);
   if (l2 && R == 1 && prec != GM_FP64) {
     void* k = gm::kernel_mixed_l2(group);
     if (k) return k;
@@ -982,6 +982,13 @@ int launch_group(gm_engine* e, int phases) {
     grp = (phases & gm::PH_APPLY) ? KGRP_FUSED_RES : KGRP_LANCZOS_RES;
   else if (e->kp.reorth > 0 && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_RO;
   else if (e->kp.mpk && grp == KGRP_LANCZOS) grp = KGRP_LANCZOS_MPK;
+  if (grp == KGRP_APPLY) {
+    // the lift, then the polynomial's passes
+    const dim3 lg((unsigned)((e->n + gm::kLiftBlock - 1) / gm::kLiftBlock), (unsigned)gm::lift_chunks(e->d));
+    GM_CUDA(e, cudaLaunchKernel(e->kfn[KGRP_LIFT], lg, dim3(gm::kLiftBlock), args, 0, e->stream));
+    e->launches++;
+    if (e->d == 0) return GM_OK;
+  }
   kp.G = e->Gk[grp];
   if (e->capturing) {
     // A captured launch replays with the same parameters, so the progress
@@ -1292,7 +1299,7 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   long long Gmax = 0;
   for (int g = 0; g < KGRP_N; ++g) {
     e->kfn[g] = pick_kernel(e->prec, e->R, g, l2k);
-    if (g == KGRP_SOLVE) continue;   // sized below
+    if (g == KGRP_SOLVE || g == KGRP_LIFT) continue;   // sized below or at the launch
     if (!e->kfn[g]) return fail(e, GM_ERR_UNSUPPORTED, "no kernel for nrhs %d", e->R);
     const bool res_grp = g == KGRP_LANCZOS_RES || g == KGRP_FUSED_RES;
     e->smem[g] = g == KGRP_DEFLATE ? 0 : stage_smem;

@@ -1586,83 +1586,151 @@ __device__ void phase_coef(const KParams& kp, const Ctx& c) {
 }
 
 // ------------------------------------------------------------------ APPLY
-// X_r += sum_i A^(d-i) V_r c_{r,i}: one lift pass P_i = V c_i (V read once),
-// then d Horner passes X = A X + P_i.
+// X_r += sum_i A^(d-i) V_r c_{r,i}: one lift pass P_i = V c_i, then d Horner
+// passes X = A X + P_i.
+//
+// The lift is row-local: the general path runs it as a kernel of its own
+// (k_lift, a thread per row and chunk of polynomial terms, no grid barrier, its
+// own registers), the resident entry points as part of theirs.  It streams
+// V; a load per Krylov vector and row in series left it latency-bound at a
+// third to a half of the memory rate, so QU vectors are loaded before their
+// products.  Measured, the whole apply: 300k-node disk mixed, degree 8, four
+// right-hand sides 1427 -> 667 us; 160^3 mixed without a polynomial, m = 100,
+// 626 -> 411; 117^3 FP64 225 -> 172; batch of 24 211 -> 178.  Three terms per
+// pass over V and exact counts: wider chunks cost more in registers than they
+// save in reads, and a guard per term computes the absent ones (117^3: 1616 us
+// with nine guarded terms).
+constexpr int kLiftTerms = 3;                                             // polynomial terms per pass over V
+template <int R> struct LiftWidth { static constexpr int value = R == 1 ? 8 : 4; };   // Krylov vectors in flight
+
+// acc[ii][r] = sum_q c_{r, i0 + ii}[q] V_q[i][r], q ascending.
+template <class Pol, int R, int IC>
+__device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, int i0, typename Pol::AT (&acc)[IC][R]) {
+  using BT = typename Pol::BT;
+  constexpr int QU = LiftWidth<R>::value;
+  const int m = kp.m, d1 = kp.d + 1;
+  const BT* v0 = reinterpret_cast<const BT*>(kp.V) + i * R;
+  const long long step = kp.n * R, c0 = (long long)R * p * d1 + i0;
+#pragma unroll
+  for (int ii = 0; ii < IC; ++ii)
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[ii][r] = Pol::zero();
+  auto add = [&](int q, const BT (&v)[R]) {
+#pragma unroll
+    for (int ii = 0; ii < IC; ++ii) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const long long ci = (c0 + (long long)r * d1 + ii) * m + q;
+        if constexpr (Pol::kMixed) {
+          const float2 cf = kp.coef_ff[ci];
+          acc[ii][r] = Pol::add(acc[ii][r], ff_mulf(ff{cf.x, cf.y}, v[r]));
+        } else {
+          acc[ii][r] = fma((double)v[r], kp.coef[ci], acc[ii][r]);
+        }
+      }
+    }
+  };
+  int q = 0;
+  for (; q + QU <= m; q += QU) {
+    BT v[QU][R];
+#pragma unroll
+    for (int u = 0; u < QU; ++u) VecIO<R>::ld(v0 + (q + u) * step, v[u]);
+#pragma unroll
+    for (int u = 0; u < QU; ++u) add(q + u, v[u]);
+  }
+  for (; q < m; ++q) {
+    BT v[R];
+    VecIO<R>::ld(v0 + q * step, v);
+    add(q, v);
+  }
+}
+
+// The lift's result for row i: P terms i0.., or without a polynomial X and S.
+template <class Pol, int R, int IC>
+__device__ __forceinline__ void lift_store(const KParams& kp, long long i, int i0, bool overwrite,
+                                           const typename Pol::AT (&acc)[IC][R]) {
+  using HT = typename Pol::HT;
+  if (kp.d == 0) {
+    double x[R], u[R], s[R];
+    if (overwrite) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) x[r] = 0.0;
+    } else {
+      VecIO<R>::ld(kp.X + i * R, x);
+    }
+    VecIO<R>::ld(kp.upd + i * R, u);
+#pragma unroll
+    for (int r = 0; r < R; ++r) { x[r] += Pol::to_d(acc[0][r]); s[r] = x[r] + u[r]; }
+    VecIO<R>::st(kp.X + i * R, x);
+    VecIO<R>::st(kp.S + i * R, s);
+    return;
+  }
+  HT* P = reinterpret_cast<HT*>(kp.P);
+#pragma unroll
+  for (int ii = 0; ii < IC; ++ii) {
+    HT hv[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) hv[r] = Pol::to_h(acc[ii][r]);
+    VecIO<R>::st(P + ((long long)(i0 + ii) * kp.n + i) * R, hv);
+  }
+}
+
+// Chunk y of the d + 1 terms: whole chunks of kLiftTerms, then single terms.
+__host__ __device__ inline int lift_chunks(int d) { return (d + 1) / kLiftTerms + (d + 1) % kLiftTerms; }
 template <class Pol, int R>
+__device__ __forceinline__ void lift_chunk(const KParams& kp, int p, long long i, int y, bool overwrite) {
+  const int full = (kp.d + 1) / kLiftTerms;
+  if (y < full) {
+    typename Pol::AT acc[kLiftTerms][R];
+    lift_row<Pol, R, kLiftTerms>(kp, p, i, y * kLiftTerms, acc);
+    lift_store<Pol, R, kLiftTerms>(kp, i, y * kLiftTerms, overwrite, acc);
+  } else {
+    typename Pol::AT acc[1][R];
+    const int i0 = full * kLiftTerms + (y - full);
+    lift_row<Pol, R, 1>(kp, p, i, i0, acc);
+    lift_store<Pol, R, 1>(kp, i, i0, overwrite, acc);
+  }
+}
+
+// 256 / 128 / 64 threads: 16,384 rows at m = 200 take 56 / 33 / 46 us (at 256
+// they fill 64 of 152 SMs); the large cases agree within 3 %.
+constexpr int kLiftBlock = 128;
+template <class Pol, int R>
+__global__ void __launch_bounds__(kLiftBlock) k_lift(KParams kp) {
+  if (*(volatile int*)kp.status != 0) return;
+  const long long i = (long long)blockIdx.x * kLiftBlock + threadIdx.x;
+  if (i >= kp.n) return;
+  int p = 0;   // the row's problem
+  if (kp.nprob > 1) {
+    int hi = kp.nprob;
+    while (hi - p > 1) {
+      const int mid = (p + hi) >> 1;
+      if (kp.prob_row0[mid] <= i) p = mid; else hi = mid;
+    }
+  }
+  lift_chunk<Pol, R>(kp, p, i, (int)blockIdx.y, (kp.phases & PH_APPLY_SET) != 0);
+}
+
+template <class Pol, int R, bool kLift>
 __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool overwrite, PassSync& ps,
                             ColStage& cs) {
-  using BT = typename Pol::BT;
   using HT = typename Pol::HT;
   using AT = typename Pol::AT;
   const long long n = kp.n;
-  const int m = kp.m, d = kp.d, d1 = d + 1;
-  const BT* V = reinterpret_cast<const BT*>(kp.V);
+  const int d = kp.d;
   HT* P = reinterpret_cast<HT*>(kp.P);
   HT* const H0 = reinterpret_cast<HT*>(kp.H0);
   HT* const H1 = reinterpret_cast<HT*>(kp.H1);
-  constexpr int IC = 3;
-  const long long sb = kp.blk_slice[c.b()], se = kp.blk_slice[c.b() + 1];
-  for (long long s = sb + c.warp(); s < se; s += c.nw()) {
-    long long i;
-    if constexpr (Pol::kDia) {
-      i = (__ldg(kp.dia_meta + s).y >> 16) >= 0 ? s * 32 + c.lane() - dia_table()[kDiaTable] : slot_row(kp, s, c.lane());
-    } else {
-      i = slot_row(kp, s, c.lane());
+  if constexpr (kLift) {
+    const long long sb = kp.blk_slice[c.b()], se = kp.blk_slice[c.b() + 1];
+    for (long long s = sb + c.warp(); s < se; s += c.nw()) {
+      const long long i = slot_row(kp, s, c.lane());
+      if (i < 0) continue;
+      for (int y = 0; y < lift_chunks(d); ++y) lift_chunk<Pol, R>(kp, g.p, i, y, overwrite);
     }
-    if (i < 0) continue;
-    for (int i0 = 0; i0 < d1; i0 += IC) {
-      AT acc[IC][R];
-#pragma unroll
-      for (int ii = 0; ii < IC; ++ii)
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[ii][r] = Pol::zero();
-      for (int q = 0; q < m; ++q) {
-        BT v[R];
-        VecIO<R>::ld(V + ((long long)q * n + i) * R, v);
-#pragma unroll
-        for (int ii = 0; ii < IC; ++ii) {
-          if (i0 + ii < d1) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              const long long ci = (((long long)R * g.p + r) * d1 + i0 + ii) * m + q;
-              if constexpr (Pol::kMixed) {
-                const float2 cf = kp.coef_ff[ci];
-                acc[ii][r] = Pol::add(acc[ii][r], ff_mulf(ff{cf.x, cf.y}, v[r]));
-              } else {
-                acc[ii][r] = fma((double)v[r], kp.coef[ci], acc[ii][r]);
-              }
-            }
-          }
-        }
-      }
-      if (d == 0) {
-        double x[R], u[R], s[R];
-        if (overwrite) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) x[r] = 0.0;
-        } else {
-          VecIO<R>::ld(kp.X + i * R, x);
-        }
-        VecIO<R>::ld(kp.upd + i * R, u);
-#pragma unroll
-        for (int r = 0; r < R; ++r) { x[r] += Pol::to_d(acc[0][r]); s[r] = x[r] + u[r]; }
-        VecIO<R>::st(kp.X + i * R, x);
-        VecIO<R>::st(kp.S + i * R, s);
-      } else {
-#pragma unroll
-        for (int ii = 0; ii < IC; ++ii) {
-          if (i0 + ii < d1) {
-            HT hv[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) hv[r] = Pol::to_h(acc[ii][r]);
-            VecIO<R>::st(P + ((long long)(i0 + ii) * n + i) * R, hv);
-          }
-        }
-      }
-    }
+    if (d == 0) return true;
+    ps.done(kp);
   }
-  if (d == 0) return true;
-  ps.done(kp);
   for (int h = 1; h <= d; ++h) {
     const HT* hin = h == 1 ? P : ((h & 1) ? H0 : H1);
     HT* hout = (h & 1) ? H1 : H0;
@@ -1693,7 +1761,7 @@ __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool 
         VecIO<R>::st(kp.X + row * R, xo);
         VecIO<R>::st(kp.S + row * R, so);
       }
-    }, &ps);
+    }, kLift || h > 1 ? &ps : nullptr);
     if (!ok) return false;
     if (h < d) ps.done(kp);
   }
@@ -1924,7 +1992,7 @@ __global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : PH == KG_SO
   }
   if ((PH & PH_APPLY) && (ph & PH_APPLY)) {
     if (!sep()) return;
-    if (!phase_apply<Pol, R>(kp, c, g, (ph & PH_APPLY_SET) != 0, ps, cs)) return;
+    if (!phase_apply<Pol, R, (PH & PH_RESIDENT) != 0>(kp, c, g, (ph & PH_APPLY_SET) != 0, ps, cs)) return;
   }
   if (PH & (PH_DEFLATE | PH_UPDATE_FKPP | PH_UPDATE_FHN)) {
     const int upd_mode = (ph & PH_UPDATE_FKPP) ? 1 : ((ph & PH_UPDATE_FHN) ? 2 : 0);

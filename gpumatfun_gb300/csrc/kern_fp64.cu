@@ -11,6 +11,7 @@ static void* group_ptr(int group) {
     case 3: return (void*)fab_kernel<Pol, R, KG_DEFLATE>;
     case 4: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_MPK>;
     case 5: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_REORTH>;
+    case 8: return (void*)k_lift<Pol, R>;
   }
   return nullptr;
 }
