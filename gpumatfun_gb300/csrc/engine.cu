@@ -949,9 +949,22 @@ int map_status(gm_engine* e, int st) {
   }
 }
 
+// The barrier counters with the status word behind them, on a line of its own.
+size_t bar_words(int nprob) { return (2 + 2 * (size_t)nprob + 31) / 32 * 32; }
+
+int clear_status(gm_engine* e) {
+  GM_CUDA(e, cudaMemsetAsync(e->kp.bar, 0, (bar_words(e->nprob) + 1) * sizeof(unsigned), e->stream));
+  return GM_OK;
+}
+
 int check_sync(gm_engine* e) {
-  GM_CUDA(e, cudaMemcpyAsync(e->h_status, e->kp.status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-  GM_CUDA(e, cudaMemcpyAsync(e->h_status + 1, e->kp.meff, sizeof(int) * e->R * e->nprob, cudaMemcpyDeviceToHost, e->stream));
+  // m_eff lies behind the status word (create_impl), except in the adjoint's
+  // second slot: one copy for both
+  const size_t nm = (size_t)e->R * e->nprob;
+  const bool together = e->kp.meff == e->kp.status + 1;
+  GM_CUDA(e, cudaMemcpyAsync(e->h_status, e->kp.status, sizeof(int) * (together ? 1 + nm : 1), cudaMemcpyDeviceToHost, e->stream));
+  if (!together)
+    GM_CUDA(e, cudaMemcpyAsync(e->h_status + 1, e->kp.meff, sizeof(int) * nm, cudaMemcpyDeviceToHost, e->stream));
   GM_CUDA(e, cudaStreamSynchronize(e->stream));
   return map_status(e, e->h_status[0]);
 }
@@ -1257,9 +1270,9 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
   // default, for a single unsorted problem without reorthogonalisation that
   // fits (plan_resident, and shared memory below).  It replaces matrix-powers
   // passes too, whose point is to halve the passes' waits.  Per Lanczos step,
-  // general path against this one: FP64 64 x 64 12.6 -> 5.0 us, 256 x 256
-  // 13.6 -> 8.6, 128 x 128 with two right-hand sides 18.9 -> 7.1, a 20k-node
-  // disk with two and degree 8 72 -> 22; mixed 256 x 256 with two 19.4 -> 11.9.
+  // general path against this one: FP64 64 x 64 12.6 -> 4.8 us, 256 x 256
+  // 13.7 -> 7.5, 128 x 128 with two right-hand sides 19.0 -> 6.8, a 20k-node
+  // disk with two and degree 8 72 -> 22; mixed 256 x 256 with two 19.5 -> 12.4.
   // Past 16 slices per SM a warp would hold several rows per lane, and the
   // general path's passes are long enough to hide most of its round trips.
   ResidentPlan plan;
@@ -1491,11 +1504,13 @@ int create_impl(const gm_create_args* a, const std::vector<ProbIn>& probs, gm_en
     if ((rc = dalloc(e, &kp.hpart, (size_t)2 * (m + 8) * R * e->G))) return rc;
     if ((rc = dalloc(e, &kp.hblk, (size_t)e->G * (m + 1) * R))) return rc;
   }
-  if ((rc = dalloc(e, &kp.bar, 2 + 2 * (size_t)np))) return rc;
-  if ((rc = dalloc(e, &kp.status, 1))) return rc;
-  if ((rc = dalloc(e, &kp.meff, PR))) return rc;
-  GM_CUDA(e, cudaMemset(kp.bar, 0, (2 + 2 * (size_t)np) * sizeof(unsigned)));
-  GM_CUDA(e, cudaMemset(kp.status, 0, sizeof(int)));
+  // Barrier counters, status and m_eff in one allocation: a call clears the
+  // first two in one memset and reads the last two in one copy (64 x 64 FP64,
+  // three synchronising calls: 441 -> 436 us).
+  if ((rc = dalloc(e, &kp.bar, bar_words(np) + 1 + PR))) return rc;
+  kp.status = reinterpret_cast<int*>(kp.bar + bar_words(np));
+  kp.meff = kp.status + 1;
+  GM_CUDA(e, cudaMemset(kp.bar, 0, (bar_words(np) + 1) * sizeof(unsigned)));
   GM_CUDA(e, cudaMemset(kp.aabb, 0, (size_t)(m + 1) * 2 * PR * sizeof(double)));
   GM_CUDA(e, cudaMemset(kp.X, 0, nR * sizeof(double)));
   GM_CUDA(e, cudaMemset(kp.Yr, 0, (size_t)m * PR * C * sizeof(double)));
@@ -1740,8 +1755,7 @@ static int set_U_common(gm_handle h, const double* U, bool on_device) {
   int rc = set_usol(h, U, on_device);
   if (rc) return rc;
   if (h->fe_cur == 0) h->fe_fwd_ok = false;   // the stored forward state is being replaced
-  GM_CUDA(h, cudaMemsetAsync(h->kp.status, 0, sizeof(int), h->stream));
-  GM_CUDA(h, cudaMemsetAsync(h->kp.bar, 0, (2 + 2 * (size_t)h->nprob) * sizeof(unsigned), h->stream));
+  if ((rc = clear_status(h))) return rc;
   h->have_V = h->have_y = h->have_coef = false;
   return launch(h, gm::PH_DEFLATE, 0);
 }
@@ -1761,8 +1775,7 @@ int gm_set_state(gm_handle h, const double* Usol_host, const double* ode_host) {
   int rc = set_usol(h, Usol_host, false, false);   // Usol as gm_get_U returned it: no column scaling
   if (rc) return rc;
   if (h->fe_cur == 0) h->fe_fwd_ok = false;
-  GM_CUDA(h, cudaMemsetAsync(h->kp.status, 0, sizeof(int), h->stream));
-  GM_CUDA(h, cudaMemsetAsync(h->kp.bar, 0, (2 + 2 * (size_t)h->nprob) * sizeof(unsigned), h->stream));
+  if ((rc = clear_status(h))) return rc;
   h->have_V = h->have_y = h->have_coef = false;
   return launch(h, gm::PH_DEFLATE, 0);
 }
