@@ -669,6 +669,66 @@ __device__ __forceinline__ bool spmv_pass(const KParams& kp, const Ctx& c, ColSt
   return true;
 }
 
+// The same products by (row, right-hand side): lane l of a warp takes row
+// l / R of the unit's 32 / R rows and right-hand side l % R, so a slice is R
+// units of work.  For the FP64 engine's Horner passes, which sum nothing over
+// the block: a lane holds one accumulator instead of R, which leaves registers
+// for four gathers in flight (by rows one at a time, two with R = 2), and a
+// block of few slices waits less for the warps that have one slice more.  The
+// FP64 pipe does the same number of warp instructions either way.
+// Disks of degree 8, us per step by rows / split: R = 2 200k nodes 114.9 /
+// 100.3, 500k 214.6 / 187.7, 700k 286.1 / 280.3; R = 4 100k 123.1 / 111.7, 300k
+// 216.3 / 194.1, 500k 343.9 / 311.2, 700k 464 / 434.  With more slices per warp
+// the staged columns and prefetched values of the other pass win (1M, 6.4
+// slices: R = 2 390 / 407, R = 4 655 / 680), hence kSplitSlices.  The mixed
+// engine is bound by FP32 issue and loses by the extra index loads (300k, R =
+// 4: 136 / 168); the apply's passes gain nothing (300k 539 / 540).
+// epi(e, r, z): element e = row R + r.
+template <int N> struct IntC { static constexpr int value = N; };
+constexpr int kSplitSlices = 5;   // slices per warp up to which it is taken
+template <class Pol, int R>
+__device__ __forceinline__ bool split_rows(const KParams& kp, const Ctx& c) {
+  if constexpr (R == 1 || Pol::kDia || Pol::kMixed) return false;
+  return kp.blk_slice[c.b() + 1] - kp.blk_slice[c.b()] <= kSplitSlices * c.nw();
+}
+template <class Pol, int R, class XT, class Epi>
+__device__ __forceinline__ bool spmv_pass_split(const KParams& kp, const Ctx& c, const XT* __restrict__ x, Epi&& epi,
+                                                PassSync* wait = nullptr) {
+  using AT = typename Pol::AT;
+  using VT = typename Pol::VT;
+  const int sb = kp.blk_slice[c.b()], nu = (kp.blk_slice[c.b() + 1] - sb) * R;
+  if (wait && !wait->before_next(kp)) return false;
+  for (int u = c.warp(); u < nu; u += c.nw()) {
+    const long long s = sb + u / R;
+    const int sl = (u % R) * (32 / R) + c.lane() / R, r = c.lane() % R;
+    const long long base = kp.slice_off[s];
+    const int len = (int)((kp.slice_off[s + 1] - base) >> 5);
+    const int* cp = kp.col + base + sl;
+    const VT* vp = reinterpret_cast<const VT*>(kp.val) + base + sl;
+    AT z = Pol::zero();
+    int jj = 0;
+    auto chunk = [&](auto width) {
+      constexpr int U = decltype(width)::value;
+      VT a[U];
+      XT xv[U][1];
+      int cc[U];
+#pragma unroll
+      for (int v = 0; v < U; ++v) { cc[v] = __ldg(cp + (jj + v) * 32); a[v] = ld_val(vp + (jj + v) * 32); }
+#pragma unroll
+      for (int v = 0; v < U; ++v) VecIO<1>::ld(x + (long long)cc[v] * R + r, xv[v]);
+#pragma unroll
+      for (int v = 0; v < U; ++v) z = Pol::acc(z, a[v], xv[v][0]);
+      jj += U;
+    };
+    while (jj + 4 <= len) chunk(IntC<4>{});
+    if (jj + 2 <= len) chunk(IntC<2>{});
+    if (jj < len) chunk(IntC<1>{});
+    const long long row = slot_row(kp, s, sl);
+    if (row >= 0) epi(row * R + r, r, Pol::norm(z));
+  }
+  return true;
+}
+
 // One row of A x read through the SELL layout without a row perm (row r is
 // lane r % 32 of slice r / 32): the halo rows of a matrix-powers pass.
 template <class Pol, int R, class XT>
@@ -1199,7 +1259,18 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
       }, nullptr, j > 0 ? Wout : nullptr);
     } else {
       // Horner pass 1: u = gamma_1 v_j + A (gamma_0 v_j); stores v_j
-      {
+      const bool split = split_rows<Pol, R>(kp, c);
+      if (split) {
+        spmv_pass_split<Pol, R, BT>(kp, c, src, [&](long long e, int r, AT z) {
+          BT sv[1], v[1];
+          VecIO<1>::ld(src + e, sv);
+          v[0] = Pol::scale_to_b(sv[0], sh.rb[r]);
+          VecIO<1>::st(Vj + e, v);
+          HT u[1];
+          u[0] = Pol::to_h(Pol::add_mul(Pol::mul(z, sh.sc[r]), sh.gr[1][r], sv[0]));
+          VecIO<1>::st(H1 + e, u);
+        });
+      } else {
         spmv_pass<Pol, R, BT>(kp, c, cs, src, [&](long long row, AT (&z)[R]) {
           if (row < 0) return;
           BT sv[R], v[R];
@@ -1246,7 +1317,13 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
         for (int h = 2; h <= d; ++h) {
           const HT* hin_h = (h & 1) ? H0 : H1;
           HT* hout = (h & 1) ? H1 : H0;
-          const bool ok = spmv_pass<Pol, R, HT>(kp, c, cs, hin_h, [&](long long row, AT (&z)[R]) {
+          const bool ok = split ? spmv_pass_split<Pol, R, HT>(kp, c, hin_h, [&](long long e, int r, AT z) {
+            BT sv[1];
+            VecIO<1>::ld(src + e, sv);
+            HT u[1];
+            u[0] = Pol::to_h(Pol::add_mul(z, sh.gr[h][r], sv[0]));
+            VecIO<1>::st(hout + e, u);
+          }, &ps) : spmv_pass<Pol, R, HT>(kp, c, cs, hin_h, [&](long long row, AT (&z)[R]) {
             if (row < 0) return;
             BT sv[R];
             VecIO<R>::ld(src + row * R, sv);
@@ -1396,8 +1473,8 @@ __device__ bool phase_lanczos(const KParams& kp, const Ctx& c, const Grp& g, Pas
 //   - alpha, beta, shifts and t_q are loaded kTriU entries ahead (two: the
 //     engine's kernels have 40 to 64 registers; m = 453 345 us, four 387 us);
 //   - the warps' systems are spread over the blocks, one warp per SM first.
-// Against one thread per system with Smith's formula on both sides of a branch
-// (FP64 phase times): m = 60 120 -> 72 us, m = 453 1010 -> 345 us.
+// Against one thread per system with Smith's formula on both sides of a branch:
+// FP64 m = 60 120 -> 55 us, m = 200 378 -> 147; mixed m = 453 1010 -> 450.
 constexpr int kTriU = 2;
 
 // x * 2^(-k) by exponent arithmetic: exact while x and the result are normal
