@@ -318,7 +318,7 @@ class Engine:
         self._check(self._lib.gm_set_U_device(self._h, ct.c_void_p(ptr)))
 
     def solve(self):
-        """Fused build_subspace + lin_sys_solves + apply_V in one launch."""
+        """build_subspace + lin_sys_solves + apply_V in one call."""
         self._check(self._lib.gm_solve(self._h))
 
     def get_solution(self) -> np.ndarray:

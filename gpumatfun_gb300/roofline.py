@@ -96,12 +96,12 @@ def deflate_bytes(s: Sizes) -> float:
 
 
 def fused_solve_bytes(s: Sizes) -> float:
-    """One fused launch: build_subspace + lin_sys_solves + apply_V."""
+    """One solve: build_subspace + lin_sys_solves + apply_V."""
     return lanczos_bytes(s) + solve_bytes(s) + apply_bytes(s)
 
 
 def fused_solve_flops(s: Sizes) -> float:
-    """Floating-point operations (an FMA counts 2) of one fused launch."""
+    """Floating-point operations (an FMA counts 2) of one solve."""
     spmv = 2.0 * s.nnz * s.R
     per_step = (s.d + 1) * spmv + 2.0 * s.n * s.R * (2 + s.d + 3)
     apply = 2.0 * s.n * s.R * s.m * (s.d + 1) + s.d * spmv

@@ -271,7 +271,7 @@ def config5_batch(nprob: int = 64, R: int = 4, seed: int = 0, lo: int = 64, hi: 
     (the monodomain's physical parameters: square of side 2.5, K_alpha = 1e-4,
     dt = 0.05, alpha = 1.5) on a 2D 5-point Dirichlet Laplacian with N^2
     interior nodes (N log-uniform in [lo, hi], A scaled by 1/h^2,
-    h = side/(N+1)), R right-hand sides each, all solved by one launch."""
+    h = side/(N+1)), R right-hand sides each, all solved by one call."""
     f = params.frac_exp(Kalpha * dt, alpha)
     out = []
     for i, N in enumerate(batch_sizes(nprob, lo, hi, seed)):
