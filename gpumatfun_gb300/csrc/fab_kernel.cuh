@@ -220,57 +220,28 @@ __device__ __forceinline__ long long slot_row(const KParams& kp, long long s, in
 }
 
 // acc[r] = sum_j A(row, col_j) x[col_j][r] over the slice row of this lane.
-// The slice's columns are walked in chunks of CH: all CH column indices and
-// values are loaded first (coalesced, read-only path), then all CH gathers of
-// x are issued, then the CH products are accumulated, so each chunk costs two
-// memory latencies instead of 2*CH.
-// Chunk width: one column index, one value and R gathered entries are live
-// per chunk element across the gathers.  What the SpMV needs is loads in
-// flight per SM, and resident warps supply them more cheaply than wide
-// chunks: every right-hand-side count runs its kernels at the residency
-// below with the chunk width that fits it.
-//   R = 1: three 512-thread blocks per SM (GM_MINB1, 42 registers), one entry
-//          per chunk; against two blocks with four entries: 3D 256^3 mixed
-//          40.6 vs 51.0 ms per solve, FP64 50.0 vs 63.6 ms, 1M-node FE disk
-//          FP64 21.2 vs 22.1 ms, mixed equal (16.5 ms), despite the spills at
-//          42 registers.  The matrix-powers and Gram-Schmidt entry points,
-//          whose passes hold more state, stay at two blocks (GM_MINB1X): the
-//          250k-node adjoint 288 vs 325 ms per gradient with three.
-//   R = 2: two blocks per SM (GM_MINB, 64 registers), two entries per chunk,
-//          the widest without spills there.
-//   R = 4: two blocks per SM (GM_MINB4), one entry per chunk; against one
-//          block with three entries at 128 registers (1M-node FE disk: mixed
-//          40.0 vs 48.7 ms per launch, FP64 58.6 vs 64.9 ms).  The mixed
-//          policy's Lanczos entry points run three blocks (GM_MINB4M): 1M-node
-//          disk 39.0 vs 40.5 ms, 64-problem batch 19.0 vs 20.3 ms, where FP64
-//          at three blocks is slower (63.1 vs 58.8 ms).
-#ifndef GM_CH1
-#define GM_CH1 1
-#endif
-#ifndef GM_CH2
-#define GM_CH2 2
-#endif
-#ifndef GM_CH4
-#define GM_CH4 1
-#endif
-#ifndef GM_CH4F
-#define GM_CH4F 1
-#endif
-template <class VT, class XT, int R>
-struct ChunkWidth {
-  static constexpr int value = R == 1 ? GM_CH1 : (R == 2 ? GM_CH2 : (sizeof(VT) == 8 ? GM_CH4 : GM_CH4F));
-};
-
-// acc[r] += aa[u] * xv[u][r] for u < N, in order.
-template <class Pol, int R, class XT, int N, int CH>
-__device__ __forceinline__ void acc_first(typename Pol::AT (&acc)[R], const typename Pol::VT (&aa)[CH],
-                                          const XT (&xv)[CH][R]) {
-#pragma unroll
-  for (int u = 0; u < N; ++u)
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], aa[u], xv[u][r]);
-}
-
+// What the SpMV needs is loads in flight per SM, and resident warps supply
+// them more cheaply than several entries per lane, each of which keeps a
+// column index, a value and R gathered entries live: every right-hand-side
+// count runs its kernels at the residency below with one entry per step.
+//   R = 1: three 512-thread blocks per SM (GM_MINB1, 42 registers); against
+//          two blocks with four entries: 3D 256^3 mixed 40.6 vs 51.0 ms per
+//          solve, FP64 50.0 vs 63.6 ms, 1M-node FE disk FP64 21.2 vs 22.1 ms,
+//          mixed equal (16.5 ms), despite the spills at 42 registers.  The
+//          matrix-powers and Gram-Schmidt entry points, whose passes hold more
+//          state, stay at two blocks (GM_MINB1X): the 250k-node adjoint 288 vs
+//          325 ms per gradient with three.
+//   R = 2: two blocks per SM (GM_MINB, 64 registers); against two / three
+//          entries, disks of degree 8, us per step: mixed 200k nodes 77 vs 87 /
+//          88, 500k 118 vs 137 / 142, 1M 240 vs 326 / 295; FP64 500k 169 vs 184 /
+//          185, 1M 322 vs 388 / 398.  Three blocks: 300k mixed 97 vs 84, FP64 128
+//          vs 114.
+//   R = 4: two blocks per SM (GM_MINB4); against one block with three entries
+//          at 128 registers (1M-node FE disk: mixed 40.0 vs 48.7 ms per launch,
+//          FP64 58.6 vs 64.9 ms).  The mixed policy's Lanczos entry points run
+//          three blocks (GM_MINB4M): 1M-node disk 39.0 vs 40.5 ms, 64-problem
+//          batch 19.0 vs 20.3 ms, where FP64 at three blocks is slower (63.1 vs
+//          58.8 ms).
 // One entry per step over a slice row: column index, value, gather, product.
 // The column source (shared-memory stage or global memory) is fixed for the
 // whole row, addresses advance by a slot column (32 entries) per step, and the
@@ -364,100 +335,22 @@ __device__ __forceinline__ void spmv_slot(const KParams& kp, long long s, int la
                                           typename Pol::AT (&acc)[R], const int* scol = nullptr,
                                           const int* colarr = nullptr) {
   using VT = typename Pol::VT;
-  constexpr int CH = ChunkWidth<VT, XT, R>::value;
   const long long base = kp.slice_off[s];
   const int len = (int)((kp.slice_off[s + 1] - base) >> 5);
-  if constexpr (CH == 1) {
-    // same products in the same order as the chunked loop below
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = Pol::zero();
-    float dl = 0.f;
-    if constexpr (Pol::kMixed) {
-      if (kp.dlo) dl = __ldg(kp.dlo + s * 32 + lane);
-    }
-    const VT* vp = reinterpret_cast<const VT*>(kp.val) + base + lane;
-    if (scol)
-      row_entries1<Pol, R, XT, true>(scol + lane, vp, len, x, dl, acc);
-    else
-      row_entries1<Pol, R, XT, false>((colarr ? colarr : kp.col) + base + lane, vp, len, x, dl, acc);
-    return;
-  }
-  // Chunks of two or more entries (two right-hand sides; tuning builds).
-  // Column indices from the shared-memory stage when the slice is staged,
-  // else from global memory, chosen by a warp-uniform branch per chunk;
-  // values from global memory (read-only path; with value prefetch they are
-  // already on their way into L2).  Measured against the two other shapes of
-  // this loop (a per-load select of the source, and one generic pointer for
-  // both): 1M FE disk FP64 44.6 vs 42.8 / 42.4 solves/s, mixed 57.1 vs 55.7;
-  // the generic pointer is faster only for FP64 on the HBM-streamed 3D
-  // matrix (17.2 vs 15.8), whose reference precision is the mixed engine
-  // (19.6 vs 19.3 here).
-  const int* gcp = (colarr ? colarr : kp.col) + base + lane;
-  const VT* vp = reinterpret_cast<const VT*>(kp.val) + base + lane;
 #pragma unroll
   for (int r = 0; r < R; ++r) acc[r] = Pol::zero();
   // Mixed engine: diagonal compensation of the FP32-stored values, c_r x_r.
-  // The engine stores every row's diagonal entry first (slice column 0), so
-  // x_r is the first chunk's first gather; pad lanes carry dl = 0.
+  // The engine stores every row's diagonal entry first (slice column 0); pad
+  // lanes carry dl = 0.
   float dl = 0.f;
   if constexpr (Pol::kMixed) {
     if (kp.dlo) dl = __ldg(kp.dlo + s * 32 + lane);
   }
-  for (int jj = 0; jj < len; jj += CH) {
-    int cc[CH];
-    VT aa[CH];
-    if (scol) {
-#pragma unroll
-      for (int u = 0; u < CH; ++u) cc[u] = jj + u < len ? scol[(jj + u) * 32 + lane] : 0;
-    } else {
-#pragma unroll
-      for (int u = 0; u < CH; ++u) cc[u] = jj + u < len ? __ldg(gcp + (long long)(jj + u) * 32) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < CH; ++u) aa[u] = jj + u < len ? ld_val(vp + (long long)(jj + u) * 32) : (VT)0;
-    XT xv[CH][R];
-#pragma unroll
-    for (int u = 0; u < CH; ++u)
-      if (jj + u < len) VecIO<R>::ld(x + (long long)cc[u] * R, xv[u]);
-    if constexpr (Pol::kMixed) {
-      if (jj == 0) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], dl, xv[0][r]);
-      }
-    }
-    // The chunk's valid products, in order.  In the guarded loop (FP64) the
-    // compiler turns the guard into a select and issues the missing products
-    // with a zero value: on a 7-column slice 8/7 of the FMAs (ncu DFMA count),
-    // which measured faster than branching to exact counts (1M FE disk 41.5
-    // vs 40.0 solves/s, 3D 17.0 vs 16.1).  The mixed engine's float-float
-    // products cost ~10 instructions each on an issue-bound kernel, so it
-    // branches to exactly the valid ones (+2-4%).
-    if constexpr (!Pol::kMixed) {
-#pragma unroll
-      for (int u = 0; u < CH; ++u)
-        if (jj + u < len) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], aa[u], xv[u][r]);
-        }
-      continue;
-    }
-    const int cnt = len - jj;
-    if (cnt >= CH) {
-      acc_first<Pol, R, XT, CH>(acc, aa, xv);
-    } else {
-      if constexpr (CH > 1) if (cnt == 1) acc_first<Pol, R, XT, 1>(acc, aa, xv);
-      if constexpr (CH > 2) if (cnt == 2) acc_first<Pol, R, XT, 2>(acc, aa, xv);
-      if constexpr (CH > 3) if (cnt == 3) acc_first<Pol, R, XT, 3>(acc, aa, xv);
-      if constexpr (CH > 4) if (cnt >= 4) {
-#pragma unroll
-        for (int u = 0; u < CH; ++u)
-          if (u < cnt) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) acc[r] = Pol::acc(acc[r], aa[u], xv[u][r]);
-          }
-      }
-    }
-  }
+  const VT* vp = reinterpret_cast<const VT*>(kp.val) + base + lane;
+  if (scol)
+    row_entries1<Pol, R, XT, true>(scol + lane, vp, len, x, dl, acc);
+  else
+    row_entries1<Pol, R, XT, false>((colarr ? colarr : kp.col) + base + lane, vp, len, x, dl, acc);
 }
 
 // A Horner / lift buffer entry as the policy's accumulator.
@@ -673,14 +566,14 @@ __device__ __forceinline__ bool spmv_pass(const KParams& kp, const Ctx& c, ColSt
 // l / R of the unit's 32 / R rows and right-hand side l % R, so a slice is R
 // units of work.  For the FP64 engine's Horner passes, which sum nothing over
 // the block: a lane holds one accumulator instead of R, which leaves registers
-// for four gathers in flight (by rows one at a time, two with R = 2), and a
+// for four gathers in flight (by rows one at a time), and a
 // block of few slices waits less for the warps that have one slice more.  The
 // FP64 pipe does the same number of warp instructions either way.
-// Disks of degree 8, us per step by rows / split: R = 2 200k nodes 114.9 /
-// 100.3, 500k 214.6 / 187.7, 700k 286.1 / 280.3; R = 4 100k 123.1 / 111.7, 300k
-// 216.3 / 194.1, 500k 343.9 / 311.2, 700k 464 / 434.  With more slices per warp
-// the staged columns and prefetched values of the other pass win (1M, 6.4
-// slices: R = 2 390 / 407, R = 4 655 / 680), hence kSplitSlices.  The mixed
+// Disks of degree 8, us per step by rows / split: R = 2 200k nodes 95.1 / 93.1,
+// 300k 113.9 / 116.4, 500k 180.7 / 171.1; R = 4 100k 123.1 / 111.7, 300k 216.3 /
+// 194.1, 500k 343.9 / 311.2, 700k 464 / 434.  With more slices per warp the
+// staged columns and prefetched values of the other pass win (1M, 6.4 slices,
+// R = 4: 655 / 680), hence kSplitSlices.  The mixed
 // engine is bound by FP32 issue and loses by the extra index loads (300k, R =
 // 4: 136 / 168); the apply's passes gain nothing (300k 539 / 540).
 // epi(e, r, z): element e = row R + r.
