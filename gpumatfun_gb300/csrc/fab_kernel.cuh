@@ -278,7 +278,9 @@ __device__ __forceinline__ void row_entries1(const int* __restrict__ cp, const t
 // so index and gather are not a chain of two loads and neighbouring lanes read
 // neighbouring entries.  DiaWidth entries are loaded before their products: six
 // with one right-hand side (160^3 mixed 86.4 us per step with three, 84.8 with
-// two, 82.1 with six), else as many as fit the registers without more spills.
+// two, 82.1 with six), else one (one / two / three or four: 500^2 FP64 with two
+// right-hand sides and degree 3 41.5 / 52.2 / 47.2 us, 400^2 mixed with two 16.7 /
+// 17.0 / 17.1, 24 grids mixed with four 54.9 / 55.8 / 56.7).
 // Against column indices, per step: 160^3 mixed 96.6 -> 82.1 us, 500^2 mixed
 // with four right-hand sides 62 -> 38, 24 grids up to 512^2 67 -> 61, 117^3
 // FP64 61.3 -> 57.3 (bound by FP64 issue), 700^2 FP64 28.4 -> 27.3.  The
@@ -286,7 +288,7 @@ __device__ __forceinline__ void row_entries1(const int* __restrict__ cp, const t
 // that its slice has.
 template <class Pol, int R>
 struct DiaWidth {
-  static constexpr int value = R == 1 ? 6 : (R == 4 && !Pol::kMixed ? 1 : 2);
+  static constexpr int value = R == 1 ? 6 : 1;
 };
 template <class Pol, int R, class XT>
 __device__ __forceinline__ void row_dia(const int* of, const typename Pol::VT* __restrict__ vp, int len,
