@@ -1897,6 +1897,17 @@ constexpr int KG_DEFLATE = PH_DEFLATE | PH_UPDATE_FKPP | PH_UPDATE_FHN;
 // registers for the entries loaded ahead (at 40 they spilled).
 constexpr int kSolveThreads = 128;
 
+// The shifted solves or the coefficients, one of them per launch.  Its grid is
+// sized by the SMs and not by the partition, so nothing here may look up the
+// tables that hold an entry per block of the partition.
+template <class Pol, int R>
+__global__ void __launch_bounds__(kSolveThreads, 3) k_solve(KParams kp) {
+  if (*(volatile int*)kp.status != 0) return;
+  const Ctx c(kp.G);
+  if (kp.phases & PH_TRISOLVE) phase_trisolve<R, Pol::kMixed>(kp, c);
+  if (kp.phases & PH_COEF) phase_coef<R>(kp, c);
+}
+
 // PH is the compile-time set of phases this entry point can run (the runtime
 // mask kp.phases selects among them); specialising on it lets the compiler
 // size registers per phase group.
@@ -1922,7 +1933,7 @@ template <class Pol, int R, int PH>
 #ifndef GM_MINB1L2
 #define GM_MINB1L2 2   // one right-hand side, mixed, matrix held in the L2 window (PolMixedL2)
 #endif
-__global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : PH == KG_SOLVE ? kSolveThreads : GM_MAXT, ((PH & PH_RESIDENT) ? 1 : PH == KG_SOLVE ? 3 : R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
+__global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : GM_MAXT, ((PH & PH_RESIDENT) ? 1 : R >= 4 ? ((Pol::kMixed && !(PH & (PH_MPK | PH_REORTH))) ? GM_MINB4M : GM_MINB4)
                                             : (R == 1 ? ((PH & (PH_MPK | PH_REORTH)) ? GM_MINB1X
                                                                                      : (Pol::kL2 ? GM_MINB1L2 : GM_MINB1))
                                                       : GM_MINB))) fab_kernel(KParams kp) {

@@ -6,7 +6,7 @@ template <class Pol, int R>
 static void* group_ptr(int group) {
   switch (group) {
     case 0: return (void*)fab_kernel<Pol, R, KG_LANCZOS>;
-    case 1: return (void*)fab_kernel<Pol, R, KG_SOLVE>;
+    case 1: return (void*)k_solve<Pol, R>;
     case 2: return (void*)fab_kernel<Pol, R, KG_APPLY>;
     case 3: return (void*)fab_kernel<Pol, R, KG_DEFLATE>;
     case 4: return (void*)fab_kernel<Pol, R, KG_LANCZOS | PH_MPK>;
