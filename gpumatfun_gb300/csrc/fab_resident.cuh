@@ -392,7 +392,8 @@ __device__ bool phase_lanczos_resident(const KParams& kp, const Ctx& c) {
   rs.init(kp);
   BT* const V = reinterpret_cast<BT*>(kp.V);
   const LanczosOut out{kp.aabb, kp.meff, c.b() == 0 && c.lane() == 0};
-  if (c.tid() <= d) sh.gam[c.tid()] = kp.gamma[c.tid()];
+  // (a block of one slice has 32 threads, a polynomial up to 33 coefficients)
+  for (int i = c.tid(); i <= d; i += c.nt()) sh.gam[i] = kp.gamma[i];
   auto read_halo = [&]() -> bool {
     const int w0 = c.nw() > R ? R : 0;   // the warps that do not reduce, or all
     if (c.warp() < w0) return true;
