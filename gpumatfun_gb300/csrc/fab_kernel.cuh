@@ -1974,6 +1974,10 @@ __global__ void __launch_bounds__((PH & PH_RESIDENT) ? kResThreads : GM_MAXT, ((
   }
   if ((PH & PH_TRISOLVE) && (ph & PH_TRISOLVE)) {
     if (!sep()) return;
+    // A build that met a non-finite value has recorded it before its barrier:
+    // the handle's results stay as they were.  (Launched by themselves, the
+    // phases after the build find the status where they start.)
+    if (__syncthreads_or(c.tid() == 0 && *(volatile int*)kp.status != 0)) return;
     phase_trisolve<R, Pol::kMixed>(kp, c);
   }
   if ((PH & PH_COEF) && (ph & PH_COEF)) {
