@@ -1380,32 +1380,11 @@ __device__ __forceinline__ double scale_exp2(double x, int k) {
   return ex > max(k, 0) ? __hiloint2double(hi - (k << 20), __double2loint(x)) : 0.0;
 }
 
-// This lane's component of 1/(a + ib), x being this lane's component (even
-// lanes a, odd lanes b).  g is scaled by 2^-e, e the exponent of its larger
-// component, so that |g|^2 lies in [1, 8); its reciprocal takes one cubically
-// convergent Newton step r (1 + h + h^2), h = 1 - d r, from the FP32
-// reciprocal instruction, whose error of about 2^-22 becomes 2^-66 before
-// rounding.
-__device__ __forceinline__ double pair_recip(double x) {
-  const unsigned full = 0xffffffffu;
-  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
-  const int em = max(ex, __shfl_xor_sync(full, ex, 1));
-  const int k = em - 1023;
-  const double xs = em == 0x7ff ? x : scale_exp2(x, k);   // Inf and NaN pass through as they are
-  const double sq = xs * xs;
-  const double d = sq + __shfl_xor_sync(full, sq, 1);
-  float rf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"((float)d));
-  const double r0 = (double)rf;
-  const double h = fma(-d, r0, 1.0);
-  const double r = fma(r0, fma(h, h, h), r0);
-  const double y = em == 0x7ff ? xs * r : scale_exp2(xs * r, k);
-  return (threadIdx.x & 1) ? -y : y;
-}
-
-// The same by Smith's formula, which never forms |g|^2: with x the larger and
-// y the smaller component, t = y / x and v = 1 / (x + y t), 1/g is (v, -t v)
-// for a larger real part and (t v, -v) otherwise.
+// This lane's component of 1/(a + ib), g being this lane's component (even
+// lanes a, odd lanes b), by Smith's formula, which never forms |g|^2: with x the
+// larger and y the smaller component, t = y / x and v = 1 / (x + y t), 1/g is
+// (v, -t v) for a larger real part and (t v, -v) otherwise.  Called by whole
+// warps, as pair_recip is.
 __device__ __forceinline__ double pair_recip_smith(double g) {
   const double o = __shfl_xor_sync(0xffffffffu, g, 1);
   const bool im = threadIdx.x & 1;
@@ -1416,6 +1395,36 @@ __device__ __forceinline__ double pair_recip_smith(double g) {
   const double v = 1.0 / fma(y, t, x);
   const double tv = t * v;
   return im ? (real_big ? -tv : -v) : (real_big ? v : tv);
+}
+
+// The same in the FP64 engine.  g is scaled by 2^-e, e the exponent of its
+// larger component, so that |g|^2 lies in [1, 8); its reciprocal takes one cubically
+// convergent Newton step r (1 + h + h^2), h = 1 - d r, from the FP32
+// reciprocal instruction, whose error of about 2^-22 becomes 2^-66 before
+// rounding.  The scaling drops subnormal components: where those may be more
+// than 2^-63 of |g| or |1/g|, and for 0, Inf and NaN, the pair takes Smith's
+// formula, which the whole warp then runs (every shuffle names all lanes).
+__device__ __forceinline__ double pair_recip(double x) {
+  const unsigned full = 0xffffffffu;
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
+  const int em = max(ex, __shfl_xor_sync(full, ex, 1));
+  const int k = em - 1023;
+  const double xs = scale_exp2(x, k);
+  const double sq = xs * xs;
+  const double d = sq + __shfl_xor_sync(full, sq, 1);
+  float rf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"((float)d));
+  const double r0 = (double)rf;
+  const double h = fma(-d, r0, 1.0);
+  const double r = fma(r0, fma(h, h, h), r0);
+  const double q = scale_exp2(xs * r, k);
+  double y = (threadIdx.x & 1) ? -q : q;
+  const bool out = em < 64 || em > 1980;
+  if (__any_sync(full, out)) {
+    const double z = pair_recip_smith(x);
+    if (out) y = z;
+  }
+  return y;
 }
 
 template <int R, bool kSmith>
