@@ -49,3 +49,28 @@ def test_zero_and_infinite_pivots(engine_lib):
     y = solve(engine_lib, [0.0, 1.0, np.inf, 2.0j], [-1.0, -1.0, -1.0, -1.0])
     assert not np.isfinite(y[0])
     assert y[1] == 1.0 and y[2] == 0.0 and y[3] == -0.5j
+
+
+def smith(a, b):
+    """1 / (a + i b) by Smith's formula, each operation rounded to FP64 (the sum
+    with its product in one rounding, as a fused multiply-add)."""
+    big = np.abs(a) >= np.abs(b)
+    x, y = np.where(big, a, b), np.where(big, b, a)
+    t = y / x
+    v = 1.0 / (x.astype(np.longdouble) + y.astype(np.longdouble) * t).astype(np.float64)
+    return np.where(big, v, t * v) - 1j * np.where(big, t * v, v)
+
+
+@pytest.mark.parametrize("spread", [(0, 0), (-10, 0), (0, -10), (-20, 20)])
+def test_error_is_no_larger_than_smiths(engine_lib, spread):
+    """Root mean square of the relative error over 30,000 pivots: the solves'
+    error follows it.  Smith's formula has about 0.6 of 2^-53."""
+    rng = np.random.default_rng(0)
+    n = 30_000
+    part = lambda e: rng.uniform(-1, 1, n) * 2.0 ** (rng.integers(-20, 20, n) if spread == (-20, 20) else e)
+    a, b = part(spread[0]), part(spread[1])
+    y = solve(engine_lib, a + 1j * b, np.full(n, -1.0))
+    g = wide(a) + 1j * wide(b)
+    rms = lambda z: float(np.sqrt(np.mean(np.abs(wide(z) * g - 1) ** 2)) * 2.0 ** 53)
+    assert rms(smith(a, b)) < 0.7
+    assert rms(y) <= rms(smith(a, b))
