@@ -511,9 +511,7 @@ __device__ __forceinline__ bool spmv_pass(const KParams& kp, const Ctx& c, ColSt
     for (; s < se; s += c.nw()) {
       const long long sn = s + c.nw();
       const int2 mn = sn < se ? __ldg(kp.dia_meta + sn) : make_int2(0, 0);
-      // (an ordinary slice without entries has nothing to fetch, and may lie at
-      // the end of the values)
-      if (kp.pf_vals && sn < se && c.lane() == 0 && (mn.y & 0xffff) != 0) {
+      if (kp.pf_vals && sn < se && c.lane() == 0) {
         tma_bulk_prefetch_l2(static_cast<const unsigned char*>(kp.val) + (long long)mn.x * 32 * kp.pf_vals,
                              (unsigned)kp.pf_vals * 32u * (unsigned)(mn.y & 0xffff));
         if (kRowB > 0 && rowpf && tab[kDiaTable] == 0 && (mn.y >> 16) >= 0)
