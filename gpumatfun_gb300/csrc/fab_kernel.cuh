@@ -22,6 +22,7 @@
 //   hpart, hblk  (Gram-Schmidt only) per-block partial dots [2][m+8][R][G]
 //                and each block's totals [G][m+1][R]
 #pragma once
+#include "dia_slices.cuh"
 #include "fab_common.cuh"
 
 namespace gm {
@@ -326,7 +327,6 @@ __device__ __forceinline__ void row_dia(const int* of, const typename Pol::VT* _
 
 // The offsets of the patterns of the block's problem and its row shift, in
 // shared memory.
-constexpr int kDiaTable = 512;
 __device__ __forceinline__ int* dia_table() {
   __shared__ int s_dia[kDiaTable + 1];
   return s_dia;
