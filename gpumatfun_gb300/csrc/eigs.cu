@@ -417,11 +417,20 @@ __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ Hin,
       __syncthreads();
     }
   }
-  // ascending order: rank of each diagonal entry
+  // ascending order: rank of each diagonal entry, by the bits as integers, an
+  // order that NaN is part of (the ranks are a permutation whatever H holds)
   __syncthreads();
+  auto key = [](double x) {
+    const long long b = __double_as_longlong(x == 0.0 ? 0.0 : x);
+    return b < 0 ? b ^ 0x7fffffffffffffffll : b;
+  };
   const double mine = H[lane][lane];
+  const long long km = key(mine);
   int rank = 0;
-  for (int j = 0; j < P; ++j) rank += H[j][j] < mine || (H[j][j] == mine && j < lane);
+  for (int j = 0; j < P; ++j) {
+    const long long kj = key(H[j][j]);
+    rank += kj < km || (kj == km && j < lane);
+  }
   if (i == 0) theta[rank] = mine;
   rank = __shfl_sync(full, rank, i);
   W[lane * P + rank] = v;
