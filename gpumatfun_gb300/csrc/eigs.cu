@@ -295,48 +295,42 @@ __global__ void k_take_cols(long long n, int k, const double* __restrict__ X, do
   }
 }
 
-// G = L L^T (Cholesky, L lower), then M = L^{-T} (so that X M has orthonormal
-// columns).  status[0] = 1 when G is not numerically positive definite (a pivot
-// at or below 1e-14 of the largest diagonal entry).
-// One block, warp i and lane j at entry (i, j): each of the 32 steps of the
-// factorisation and of the substitution is one update of every entry (one
-// warp did them entry by entry, 92 us).
-__global__ void __launch_bounds__(1024) k_chol_inv(const double* __restrict__ Gin, double* __restrict__ M,
-                                                   int* __restrict__ status) {
+// One warp: G = L L^T (Cholesky, L lower), then M = L^{-T} (so that X M has
+// orthonormal columns).  status[0] = 1 when G is not numerically positive
+// definite (a pivot at or below 1e-14 of the largest diagonal entry).
+__global__ void k_chol_inv(const double* __restrict__ Gin, double* __restrict__ M, int* __restrict__ status) {
   __shared__ double L[P][P + 1];
   __shared__ double Li[P][P + 1];
   __shared__ int bad;
-  const int lane = threadIdx.x & 31, i = threadIdx.x >> 5;
-  double a = Gin[threadIdx.x];
-  L[i][lane] = a;
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
+  const int lane = threadIdx.x;
+  for (int i = 0; i < P; ++i) L[i][lane] = Gin[i * P + lane];
+  if (lane == 0) bad = 0;
+  __syncwarp();
   double dmax = 0.0;
-  for (int t = 0; t < P; ++t) dmax = fmax(dmax, L[t][t]);
-  __syncthreads();
+  for (int i = 0; i < P; ++i) dmax = fmax(dmax, L[i][i]);
   for (int k = 0; k < P; ++k) {
-    if (i == k && lane == k) {
-      if (!(a > 1e-14 * dmax)) bad = 1;
-      a = sqrt(fmax(a, 1e-300));
-      L[k][k] = a;
+    if (lane == 0) {
+      const double d = L[k][k];
+      if (!(d > 1e-14 * dmax)) bad = 1;
+      L[k][k] = sqrt(fmax(d, 1e-300));
     }
-    __syncthreads();
-    if (i > k && lane == k) {
-      a /= L[k][k];
-      L[i][k] = a;
-    }
-    __syncthreads();
-    if (i > k && lane > k && lane <= i) a -= L[i][k] * L[lane][k];
+    __syncwarp();
+    if (lane > k) L[lane][k] /= L[k][k];
+    __syncwarp();
+    for (int j = k + 1; j < P; ++j)
+      if (lane >= j) L[lane][j] -= L[lane][k] * L[j][k];
+    __syncwarp();
   }
-  // L^{-1} by forward substitution, row t of all columns at once
-  double s = i == lane ? 1.0 : 0.0;
-  for (int t = 0; t < P; ++t) {
-    if (i == t) Li[t][lane] = t >= lane ? s / L[t][t] : 0.0;
-    __syncthreads();
-    if (i > t) s -= L[i][t] * Li[t][lane];
+  // column `lane` of L^{-1} by forward substitution
+  for (int i = 0; i < P; ++i) {
+    double s = i == lane ? 1.0 : 0.0;
+    for (int t = 0; t < i; ++t) s -= L[i][t] * Li[t][lane];
+    Li[i][lane] = i >= lane ? s / L[i][i] : 0.0;
+    __syncwarp();
   }
-  M[threadIdx.x] = Li[lane][i];   // M[i][j] = (L^{-1})[j][i]
-  if (threadIdx.x == 0) status[0] = bad;
+  // M[i][j] = (L^{-1})[j][i]
+  for (int i = 0; i < P; ++i) M[i * P + lane] = Li[lane][i];
+  if (lane == 0) status[0] = bad;
 }
 
 // Eigendecomposition of the symmetric 32 x 32 H by cyclic Jacobi rotations
@@ -511,7 +505,7 @@ struct Solver {
   int cholqr2(double* X, double* tmp) {
     for (int pass = 0; pass < 2; ++pass) {
       if (gram(X, X) != cudaSuccess) return -1;
-      k_chol_inv<<<1, 1024>>>(small, small + P * P, status);
+      k_chol_inv<<<1, 32>>>(small, small + P * P, status);
       int bad = 0;
       if (cudaMemcpy(&bad, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
       if (bad) return 1;
