@@ -1943,10 +1943,11 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_solve(KParams kp) {
 #ifndef GM_MINB
 #define GM_MINB 2
 #endif
-template <class Pol, int R, int PH>
 #ifndef GM_MAXT
 #define GM_MAXT 512
 #endif
+static_assert(GM_MAXT <= ReduceBuf<1>::kCap, "a block's sums are staged in kCap words");
+template <class Pol, int R, int PH>
 #ifndef GM_MINB4
 #define GM_MINB4 2   // resident 512-thread blocks per SM for four right-hand sides
 #endif
