@@ -837,7 +837,7 @@ void window_release(int dev) {
 
 // l2: a mixed engine's matrix is held in the L2 persisting window; one
 // right-hand side then runs the SpMV groups compiled for two resident blocks
-// per SM (gm::PolMixedL2, no register spills).
+// per SM (gm::PolMixedL2).
 void* pick_kernel(int prec, int R, int group, bool l2) {
   if (group == KGRP_LANCZOS_RES || group == KGRP_FUSED_RES) return gm::kernel_resident(prec == GM_FP64, R, group == KGRP_FUSED_RES);
   if (l2 && R == 1 && prec != GM_FP64) {

@@ -206,14 +206,16 @@ struct PolMixed {
 };
 
 // The mixed arithmetic for one-right-hand-side kernels compiled at two
-// resident 512-thread blocks per SM (64 registers, no spills) instead of
-// three (40 registers).  Mixed engines whose matrix is held in the L2
-// persisting window use them: there the spill frames of the 40-register build
-// compete with the vectors for the L2 left beside the window (1M-node FE disk:
-// 13.9 vs 14.5 ms per solve), while a matrix streamed from HBM wants the third
-// block's loads in flight (3D 256^3: 44.6 vs 37.8 ms with two blocks).  The
-// FP64 engine, which spills little at 40 registers, measured slower with two
-// blocks on the same L2-held disk (21.2 vs 19.2 ms) and has no such variant.
+// resident 512-thread blocks per SM (64 registers) instead of three (40; neither
+// spills).  Mixed engines whose matrix is held in the L2 persisting window use
+// them: there two blocks fill as many issue slots as three (30 %, L1 and L2 hits
+// alike on a disk of 500k nodes), and the third adds to the waits at the block
+// barriers (11 against 19 warps per issue).  Two / three blocks, ms a solve: disks
+// of degree 8, 200k nodes 5.75 / 5.74, 500k 8.39 / 9.13, 1M 13.35 / 15.85; grids
+// 700^2 1.29 / 1.35, 1300^2 2.31 / 2.38, 1000^2 of degree 3 3.88 / 3.98.  A matrix
+// streamed from HBM wants the third block's loads in flight: 160^3 9.57 / 8.72, a
+// disk of 1.6M nodes 24.2 / 23.7.  So does the FP64 engine on disks, held in L2
+// or not (500k 10.67 / 9.78, 1M 18.5 / 17.0), and has no such variant.
 struct PolMixedL2 : PolMixed { static constexpr bool kL2 = true; };
 
 // The same arithmetic for matrices whose slices are mostly diagonals: every
@@ -326,10 +328,13 @@ struct GridBar {
   unsigned long long timeout_ns;
 
   // One thread's arrival for its block, and its wait for the others (the
-  // block's stores are ordered before it by a block barrier).  A block that
-  // records an error leaves and never arrives again, so the others find the
-  // status in their next wait: no read of it after a wait that succeeded (a
-  // round trip per barrier).
+  // block's stores are ordered before it by a block barrier).  A block whose
+  // wait ran out leaves and never arrives again, so the others find the status
+  // in their next wait: no read of it after a wait that succeeded (a round trip
+  // per barrier).  Two errors do not stop the block that records them and need
+  // not: a non-finite value, whose launch computes on and whose later phases
+  // look at the status before they write results, and a staged copy that timed
+  // out, whose slice is read from global memory instead.
   __device__ bool arrive_and_wait() const {
     if (nblocks <= 1) return true;
     bool ok = true;

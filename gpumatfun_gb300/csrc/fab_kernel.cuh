@@ -225,13 +225,13 @@ __device__ __forceinline__ long long slot_row(const KParams& kp, long long s, in
 // them more cheaply than several entries per lane, each of which keeps a
 // column index, a value and R gathered entries live: every right-hand-side
 // count runs its kernels at the residency below with one entry per step.
-//   R = 1: three 512-thread blocks per SM (GM_MINB1, 42 registers); against
-//          two blocks with four entries: 3D 256^3 mixed 40.6 vs 51.0 ms per
-//          solve, FP64 50.0 vs 63.6 ms, 1M-node FE disk FP64 21.2 vs 22.1 ms,
-//          mixed equal (16.5 ms), despite the spills at 42 registers.  The
-//          matrix-powers and Gram-Schmidt entry points, whose passes hold more
-//          state, stay at two blocks (GM_MINB1X): the 250k-node adjoint 288 vs
-//          325 ms per gradient with three.
+//   R = 1: three 512-thread blocks per SM (GM_MINB1, 40 registers, no spills);
+//          against two blocks, ms a solve: 160^3 mixed 8.72 vs 9.57, disks of
+//          degree 8 FP64 500k nodes 9.78 vs 10.67, 1M 17.0 vs 18.5 (160^3 FP64 12.3
+//          vs 12.0); a mixed engine's matrix held in L2 is the exception
+//          (PolMixedL2).  The matrix-powers and Gram-Schmidt entry points, whose
+//          passes hold more state, stay at two blocks (GM_MINB1X): the 250k-node
+//          adjoint 288 vs 325 ms per gradient with three.
 //   R = 2: two blocks per SM (GM_MINB, 64 registers); against two / three
 //          entries, disks of degree 8, us per step: mixed 200k nodes 77 vs 87 /
 //          88, 500k 118 vs 137 / 142, 1M 240 vs 326 / 295; FP64 500k 169 vs 184 /

@@ -1,6 +1,7 @@
 // Entry points whose Lanczos phase keeps the problem on chip
 // (fab_resident.cuh): the Lanczos group and the fused solve, both precisions.
-// One block per SM, so every phase compiles for 128 registers.
+// One block of up to 640 threads per SM: the phases have up to 96 registers
+// (they take 80 to 96, without spills).
 #include "fab_kernel.cuh"
 
 namespace gm {

@@ -7,8 +7,8 @@
 // latency-critical path where cudaMalloc's implicit device-wide
 // synchronisation is not acceptable.  They hand over their own device
 // buffers for the inputs and the outputs; the only extra memory the solve
-// needs, the table of reciprocal Schur complements 1/g_q (strided by four
-// doubles per system entry) and nrhs m_eff slots, lives in the file-scope
+// needs, the table of 1/g_0 and beta_q / g_q of the Schur complements g_q
+// (strided by four doubles per system entry) and nrhs m_eff slots, lives in the file-scope
 // array g_noalloc_scratch below, which every GPU that loads this library
 // holds until the process exits.
 //

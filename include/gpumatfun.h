@@ -134,7 +134,10 @@ typedef struct gm_create_args {
                                   pass (halo rows recomputed per block, the level
                                   in between in shared memory), where it applies:
                                   one problem, no sigma sorting, the vector fits
-                                  shared memory; 0 = one level per pass            */
+                                  shared memory, and not a small problem kept on
+                                  chip (gm_info_ex [19]), whose passes wait less
+                                  (gm_info [13] says whether they run); 0 = one
+                                  level per pass                                   */
   int reorth;                  /* Gram-Schmidt reorthogonalisation of every new
                                   Lanczos vector against the stored basis, with
                                   FP64 dot products: 0 = none (the reference's
@@ -263,8 +266,9 @@ int gm_get_solution(gm_handle h, double* dst);
  * handle's stream (no host synchronisation unless sync_mode is set). */
 int gm_get_solution_device(gm_handle h, double* dst_dev);
 
-/* One f(A)b evaluation in a single persistent launch: build_subspace,
- * lin_sys_solves and apply_V fused; then X + update is available. */
+/* One f(A)b evaluation: build_subspace, lin_sys_solves and apply_V, one launch
+ * per phase on the handle's stream (one in all for small problems); then
+ * X + update is available. */
 int gm_solve(gm_handle h);
 
 /* End to end with host buffers: set_U(b_host), gm_solve, solution -> x_host. */
