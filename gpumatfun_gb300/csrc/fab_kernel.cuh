@@ -1603,13 +1603,6 @@ __device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, 
   using BT = typename Pol::BT;
   constexpr int QU = LiftWidth<R>::value;
   const int m = kp.m, d1 = kp.d + 1;
-  // The build stops where the last column does, and writes no vectors past
-  // that: they may hold anything, NaN included, which zero coefficients do not
-  // take out.
-  int mv = 0;
-#pragma unroll
-  for (int r = 0; r < R; ++r) mv = max(mv, kp.meff[R * p + r]);
-  mv = min(mv, m);
   const BT* v0 = reinterpret_cast<const BT*>(kp.V) + i * R;
   const long long step = kp.n * R, c0 = (long long)R * p * d1 + i0;
 #pragma unroll
@@ -1632,14 +1625,14 @@ __device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, 
     }
   };
   int q = 0;
-  for (; q + QU <= mv; q += QU) {
+  for (; q + QU <= m; q += QU) {
     BT v[QU][R];
 #pragma unroll
     for (int u = 0; u < QU; ++u) VecIO<R>::ld(v0 + (q + u) * step, v[u]);
 #pragma unroll
     for (int u = 0; u < QU; ++u) add(q + u, v[u]);
   }
-  for (; q < mv; ++q) {
+  for (; q < m; ++q) {
     BT v[R];
     VecIO<R>::ld(v0 + q * step, v);
     add(q, v);
