@@ -1597,9 +1597,11 @@ __device__ void phase_coef(const KParams& kp, const Ctx& c) {
 constexpr int kLiftTerms = 3;                                             // polynomial terms per pass over V
 template <int R> struct LiftWidth { static constexpr int value = R == 1 ? 8 : 4; };   // Krylov vectors in flight
 
-// acc[ii][r] = sum_q c_{r, i0 + ii}[q] V_q[i][r], q ascending.
+// acc[ii][r] = sum_q c_{r, i0 + ii}[q] V_q[i][r] over the first mv vectors, q
+// ascending.
 template <class Pol, int R, int IC>
-__device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, int i0, typename Pol::AT (&acc)[IC][R]) {
+__device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, int i0, int mv,
+                                         typename Pol::AT (&acc)[IC][R]) {
   using BT = typename Pol::BT;
   constexpr int QU = LiftWidth<R>::value;
   const int m = kp.m, d1 = kp.d + 1;
@@ -1625,14 +1627,14 @@ __device__ __forceinline__ void lift_row(const KParams& kp, int p, long long i, 
     }
   };
   int q = 0;
-  for (; q + QU <= m; q += QU) {
+  for (; q + QU <= mv; q += QU) {
     BT v[QU][R];
 #pragma unroll
     for (int u = 0; u < QU; ++u) VecIO<R>::ld(v0 + (q + u) * step, v[u]);
 #pragma unroll
     for (int u = 0; u < QU; ++u) add(q + u, v[u]);
   }
-  for (; q < m; ++q) {
+  for (; q < mv; ++q) {
     BT v[R];
     VecIO<R>::ld(v0 + q * step, v);
     add(q, v);
@@ -1672,16 +1674,16 @@ __device__ __forceinline__ void lift_store(const KParams& kp, long long i, int i
 // Chunk y of the d + 1 terms: whole chunks of kLiftTerms, then single terms.
 __host__ __device__ inline int lift_chunks(int d) { return (d + 1) / kLiftTerms + (d + 1) % kLiftTerms; }
 template <class Pol, int R>
-__device__ __forceinline__ void lift_chunk(const KParams& kp, int p, long long i, int y, bool overwrite) {
+__device__ __forceinline__ void lift_chunk(const KParams& kp, int p, long long i, int y, int mv, bool overwrite) {
   const int full = (kp.d + 1) / kLiftTerms;
   if (y < full) {
     typename Pol::AT acc[kLiftTerms][R];
-    lift_row<Pol, R, kLiftTerms>(kp, p, i, y * kLiftTerms, acc);
+    lift_row<Pol, R, kLiftTerms>(kp, p, i, y * kLiftTerms, mv, acc);
     lift_store<Pol, R, kLiftTerms>(kp, i, y * kLiftTerms, overwrite, acc);
   } else {
     typename Pol::AT acc[1][R];
     const int i0 = full * kLiftTerms + (y - full);
-    lift_row<Pol, R, 1>(kp, p, i, i0, acc);
+    lift_row<Pol, R, 1>(kp, p, i, i0, mv, acc);
     lift_store<Pol, R, 1>(kp, i, i0, overwrite, acc);
   }
 }
@@ -1702,7 +1704,7 @@ __global__ void __launch_bounds__(kLiftBlock) k_lift(KParams kp) {
       if (kp.prob_row0[mid] <= i) p = mid; else hi = mid;
     }
   }
-  lift_chunk<Pol, R>(kp, p, i, (int)blockIdx.y, (kp.phases & PH_APPLY_SET) != 0);
+  lift_chunk<Pol, R>(kp, p, i, (int)blockIdx.y, kp.m, (kp.phases & PH_APPLY_SET) != 0);
 }
 
 template <class Pol, int R, bool kLift>
@@ -1716,11 +1718,15 @@ __device__ bool phase_apply(const KParams& kp, const Ctx& c, const Grp& g, bool 
   HT* const H0 = reinterpret_cast<HT*>(kp.H0);
   HT* const H1 = reinterpret_cast<HT*>(kp.H1);
   if constexpr (kLift) {
+    // (the vectors past m_eff of every column stay out: see clear_unwritten)
+    int mv = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) mv = max(mv, kp.meff[R * g.p + r]);
     const long long sb = kp.blk_slice[c.b()], se = kp.blk_slice[c.b() + 1];
     for (long long s = sb + c.warp(); s < se; s += c.nw()) {
       const long long i = slot_row(kp, s, c.lane());
       if (i < 0) continue;
-      for (int y = 0; y < lift_chunks(d); ++y) lift_chunk<Pol, R>(kp, g.p, i, y, overwrite);
+      for (int y = 0; y < lift_chunks(d); ++y) lift_chunk<Pol, R>(kp, g.p, i, y, mv, overwrite);
     }
     if (d == 0) return true;
     ps.done(kp);
@@ -1919,7 +1925,39 @@ constexpr int KG_DEFLATE = PH_DEFLATE | PH_UPDATE_FKPP | PH_UPDATE_FHN;
 // registers for the entries loaded ahead (at 40 they spilled).
 constexpr int kSolveThreads = 128;
 
-// The shifted solves or the coefficients, one of them per launch.  Its grid is
+// Zeros in the Krylov vectors that a build left unwritten because every column
+// of a problem broke down.  The lift reads all m, and what they held before
+// (fresh memory, or NaN of a failed build) would come through its zero
+// coefficients.  It is done here, where nothing is tight: an end to the lift's
+// loop at m_eff cost the batch of 24 1 %, and these lines after the Lanczos loop
+// made one of its entry points spill.  (In the resident one-launch solve it is
+// the other way round: 64 x 64 takes 432 us with the loop's end at m_eff and 446
+// with these lines.)
+template <class Pol, int R>
+__device__ void clear_unwritten(const KParams& kp, const Ctx& c) {
+  using BT = typename Pol::BT;
+  const int m = kp.m, np = kp.nprob > 0 ? kp.nprob : 1;
+  auto written = [&](int p) {
+    int mv = 0;
+    for (int r = 0; r < R; ++r) mv = max(mv, kp.meff[R * p + r]);
+    return mv;
+  };
+  bool any = false;
+  for (int p = c.tid(); p < np; p += c.nt()) any = any || written(p) < m;
+  if (!__syncthreads_or(any)) return;
+  BT* const V = reinterpret_cast<BT*>(kp.V);
+  BT z[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) z[r] = (BT)0;
+  for (int p = 0; p < np; ++p) {
+    const long long r0 = kp.nprob > 0 ? kp.prob_row0[p] : 0, r1 = kp.nprob > 0 ? kp.prob_row0[p + 1] : kp.n;
+    for (int q = written(p); q < m; ++q)
+      for (long long i = r0 + c.gt(); i < r1; i += c.tt()) VecIO<R>::st(V + ((long long)q * kp.n + i) * R, z);
+  }
+}
+
+// The shifted solves or the coefficients, one of them per launch; the latter
+// always comes between a build and its apply.  Its grid is
 // sized by the SMs and not by the partition, so nothing here may look up the
 // tables that hold an entry per block of the partition.
 template <class Pol, int R>
@@ -1927,7 +1965,10 @@ __global__ void __launch_bounds__(kSolveThreads, 3) k_solve(KParams kp) {
   if (*(volatile int*)kp.status != 0) return;
   const Ctx c(kp.G);
   if (kp.phases & PH_TRISOLVE) phase_trisolve<R, Pol::kMixed>(kp, c);
-  if (kp.phases & PH_COEF) phase_coef<R>(kp, c);
+  if (kp.phases & PH_COEF) {
+    clear_unwritten<Pol, R>(kp, c);
+    phase_coef<R>(kp, c);
+  }
 }
 
 // PH is the compile-time set of phases this entry point can run (the runtime

@@ -26,11 +26,11 @@ def body(source: str, head: str) -> str:
 
 @pytest.mark.parametrize("unit", ["kern_fp64.cu", "kern_mixed.cu"])
 def test_reads_no_table_of_the_partition(unit):
-    """The kernel registered for the solves, and the two phases it calls, use
+    """The kernel registered for the solves, and what it calls, use
     no block tables (blk_*, prob_blk0, Grp, which reads both)."""
     kernel = re.search(r"case 1: return \(void\*\)(\w+)<", open(os.path.join(CSRC, unit)).read()).group(1)
     source = open(os.path.join(CSRC, "fab_kernel.cuh")).read()
-    for head in (r"\b%s\(KParams kp\)" % kernel, r"\bphase_trisolve\(", r"\bphase_coef\("):
+    for head in (r"\b%s\(KParams kp\)" % kernel, r"\bclear_unwritten\(", r"\bphase_trisolve\(", r"\bphase_coef\("):
         assert not re.search(r"\bGrp\b|\bgroup_bar\b|\bblk_\w+|\bprob_blk0\b", body(source, head)), head
 
 
