@@ -21,7 +21,8 @@ def rel(a, b):
 @pytest.mark.parametrize("store_basis,matrix_powers", [(True, 1), (False, 1), (True, 0)])
 def test_gradient_on_the_general_path(engine_lib, precision, tol_b, tol_k, store_basis, matrix_powers):
     """Against the same formula in FP64 on the oracle's Krylov state, at a kappa
-    other than the one the engine was created with."""
+    other than the one the engine was created with.  20 nodes: the lift takes eight
+    to a block, and the last block has four."""
     mesh = problems.disk_mesh(1500, seed=4)
     cent = mesh.nodes[mesh.tris].mean(axis=1)
     kappa0 = np.exp(problems.gaussian_random_field(cent, sigma=1.0, ell=0.1, seed=5))
@@ -29,7 +30,7 @@ def test_gradient_on_the_general_path(engine_lib, precision, tol_b, tol_k, store
     n = int((~mesh.boundary).sum())
     rng = np.random.default_rng(6)
     b, g = rng.random(n), rng.random(n) - 0.5
-    op = adjoint.FracFEOperator(mesh, kappa0, m=30, C=24, degree=5, store_basis=store_basis, precision=precision,
+    op = adjoint.FracFEOperator(mesh, kappa0, m=30, C=20, degree=5, store_basis=store_basis, precision=precision,
                                 matrix_powers=matrix_powers, threads=128)
     info = op.engine.info()
     assert not info["resident"] and info["matrix_powers"] == matrix_powers and info["grid_blocks"] > 8
