@@ -811,11 +811,31 @@ __device__ __forceinline__ void step_beta(LanczosScalars<Pol, R>& sh, const KPar
   const bool normal = hi >= 0x00100000 && hi < 0x7ff00000;
   double rb, bn;
   if (normal && !Pol::kMixed) {
-    // 1/sqrt(tot), and sqrt(tot) with its residual corrected (the mixed engine
-    // keeps the bits of the square root and the division)
-    rb = rsqrt(tot);
-    const double b0 = tot * rb;
-    bn = fma(fma(-b0, b0, tot), 0.5 * rb, b0);
+    // sqrt(tot) and its reciprocal by Newton's iteration from the FP32
+    // instruction, y = 1/sqrt(t) with an error of about 2^-22 (t: tot scaled by an
+    // even power of two into [1, 4)): twice b + (t - b^2) y / 2, then y (1 + h + h^2)
+    // with h = 1 - b y; eight FP64 instructions.  (The mixed engine keeps the
+    // bits of the square root and the division.)  The reciprocal is that of the
+    // rounded b, as a division gives it: with rsqrt(tot) itself, beta_j v_j missed
+    // w_j by 0.49 of 2^-53 root mean square instead of 0.40, and solutions that
+    // Lanczos rounding decides lost as much (45^3, m = 60, 250 right-hand sides:
+    // 1.0e-12 against 8.2e-13); rsqrt and the corrections after it took 64 x 64
+    // 434 us, this 432.
+    const int ex = (((hi >> 20) - 1023) & ~1) * 0x100000;
+    const int lo = __double2loint(tot);
+    const double t = __hiloint2double(hi - ex, lo);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;"
+        : "=f"(yf) : "f"(__int_as_float(((hi - ex - 0x38000000) << 3) | (int)((unsigned)lo >> 29))));
+    const int yb = __float_as_int(yf), yh = (yb >> 3) + 0x38000000;
+    const double y = __hiloint2double(yh, yb << 29), half_y = __hiloint2double(yh - 0x100000, yb << 29);
+    double b = t * y;
+    b = fma(fma(-b, b, t), half_y, b);
+    b = fma(fma(-b, b, t), half_y, b);
+    const double h = fma(-b, y, 1.0);
+    const double r = fma(y, fma(h, h, h), y);
+    bn = __hiloint2double(__double2hiint(b) + ex / 2, __double2loint(b));
+    rb = __hiloint2double(__double2hiint(r) - ex / 2, __double2loint(r));
   } else {
     bn = sqrt(tot);
     rb = 1.0 / bn;

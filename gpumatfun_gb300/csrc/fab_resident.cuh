@@ -18,8 +18,8 @@
 //     side waits for beta.
 // A warp's FP64 instruction holds its scheduler for 64 cycles whatever its
 // active lanes, so in the FP64 engine the sums run on the integer pipe
-// (warp_fixed_sum), 1/beta and beta come from one rsqrt, and the scalars of a
-// step are formed by different lanes at once.
+// (warp_fixed_sum), beta and 1/beta come from one FP32 reciprocal square root,
+// and the scalars of a step are formed by different lanes at once.
 //
 // The mixed engine stores its Lanczos vectors in FP32, and a last-bit change of
 // alpha or beta flips roundings there that a long recurrence amplifies to
